@@ -14,6 +14,7 @@
 #include "cmc_capi_internal.hpp"
 #include "cmc_engine.cuh"
 #include "cmc_hostcore.hpp"
+#include "cmc_lanes.cuh"
 
 namespace cmc {
 
@@ -25,6 +26,8 @@ template <typename MapT, typename BinT>
 __global__ void cmc_engine_pooled(const EngineArgs a);
 template <typename MapT, typename BinT, bool WIDE, bool SMEMSLOTS>
 __global__ void cmc_engine_fused(const __grid_constant__ FusedArgs f);
+template <bool NARROW, bool WIDE>
+__global__ void cmc_lanes(const LaneArgs a);
 __global__ void cmc_compact_failures(const uint32_t* bits, uint64_t nbits, uint32_t value_base,
                                      uint32_t* out, uint32_t* count, uint64_t cap,
                                      const unsigned long long* nbits_dev);
@@ -37,6 +40,15 @@ thread_local std::string g_thread_error;
 
 
 uint32_t round_up(uint32_t x, uint32_t a) { return (x + a - 1) / a * a; }
+
+// What a launch that runs in the lane engine adds to its plan's text.
+std::string lanes_text(const LanePlan& lp) {
+    if (!lp.warps) return "";
+    char buf[96];
+    snprintf(buf, sizeof buf, " -> engine=lanes warps=%u lanes_per_warp=%u region=%llu", lp.warps, lp.share,
+             (unsigned long long)lp.region_bytes);
+    return buf;
+}
 
 }  // namespace
 
@@ -299,6 +311,102 @@ int Ctx::plan(const std::vector<Job>& jobs, Plan& pl) {
     return CMC_OK;
 }
 
+namespace {
+
+// Expected number of (item, copy) buckets the lane engine evaluates in one
+// trial: every probe of a random walk meets an empty bin with probability
+// 1 - load, so filling B bins up to t takes -B ln(1 - t/B) distinct buckets
+// (simulated at t = 1024: 1,688 of 1,688 at B = 1536, 2,136 at B = 1250).
+// With k = 2 a walk fails soon after half of the bins are full.
+double lane_evaluations(const Job& j) {
+    const double b = j.buckets, cand = double(j.pnum) * j.k;
+    const double t = j.k == 2 ? std::min<double>(j.pnum, 0.55 * b) : double(j.pnum);
+    return t < 0.999 * b ? std::min(cand, -b * std::log(1.0 - t / b)) : cand;
+}
+
+}  // namespace
+
+// The lane engine's form of a launch, or warps == 0 where the group engine
+// (whose plan is `group`) runs it.  Both sides are estimated in SM cycles:
+//   lanes: a trial is a chain of P passes (evaluations x cycle-walking, +8 %
+//     for passes a BGH25 lane sits out, +2 % for DRRT18), and W warps make a
+//     pass in 8,000 + 740 W cycles (latency of 80 dependent AES rounds, then
+//     960 shared-memory wavefronts per warp); a launch ends with its slowest
+//     trial.  15 % more with 64-bit domains.
+//   group: AES blocks over the measured 0.19-0.21 blocks per cycle and SM
+//     (0.135 with 64-bit domains, 0.125-0.15 beside walks over global slots), 500-3,000 cycles of set-up per trial, or its
+//     walks over the slots, whichever takes longer, and one trial's latency.
+// The constants are fitted to 160 launches drawn over t = 3..14,000, N =
+// 2^8..2^32, k = 2..4, both modes, 2^2..2^20 trials (B200): the choice is within
+// 2 % of the better engine on average.  At t = 64, N = 2^16, 2^20 trials: 34.1
+// ms in the group engine, 18.9 in lanes; at 4,000 trials 0.25 against 0.9.
+LanePlan Ctx::plan_lanes(const std::vector<Job>& jobs, const Plan& group) const {
+    LanePlan lp;
+    const bool forced_group = force_wg || force_ng || force_global_slots || force_walkers ||
+                              force_walker_ctas >= 0 || force_isolate >= 0 || force_method >= 0 ||
+                              force_pool >= 0 || max_slots_per_group != 8 || map_chains || fill_blocks;
+    if (force_lanes == 0 || (force_lanes < 0 && forced_group)) return lp;
+    uint64_t count = 0;
+    for (const Job& j : jobs) count += j.count;
+    if (force_lanes < 0 && count < 16ull * sms) return lp;  // far below every launch that gains
+    const bool wide_domain = group.variant == 2;
+    double trials = 0, max_b = 0, passes = 0, longest = 0;  // passes: of all trials
+    double spread = 0;  // relative spread of a trial's passes
+    double produce = 0, walk = 0, latency = 0;
+    for (const Job& j : jobs) {
+        const double n = j.count, cw = std::ldexp(1.0, 2 * int(j.half_bits)) / double(j.domain);
+        const double cand = double(j.pnum) * j.k * cw;
+        trials += n;
+        max_b = std::max<double>(max_b, j.buckets);
+        const double e = lane_evaluations(j);
+        const double p = e * cw * (j.mode == CMC_MODE_BGH25 ? 1.08 : 1.02);
+        spread += n * (jobs.size() > 1 ? 0.5 : (j.mode == CMC_MODE_BGH25 ? 2.0 : 1.1) / std::sqrt(std::max(1.0, e)));
+        passes += n * p;
+        longest = std::max(longest, p + 3.0 * std::sqrt(p) + 6.0);
+        const double build = j.method == kMethodDirect ? 8.0 * cand : 8.0 * std::ldexp(1.0, int(j.half_bits));
+        const double rate = wide_domain ? 0.135 : group.pool_stage ? 0.21 : group.slots_smem ? 0.19
+                            : j.method == kMethodCache ? 0.19 : j.method == kMethodGCache ? 0.15 : 0.125;
+        const double lookups = j.method == kMethodCache ? cand : j.method == kMethodGCache ? 1.5 * cand : 0.0;
+        produce += n * ((2.0 + build) / rate + lookups + (wide_domain ? 3000.0 : group.pool_stage ? 500.0 : 600.0));
+        const double probes = (j.mode == CMC_MODE_BGH25 ? 2.4 : 1.75) * j.pnum * (j.k == 2 ? 0.8 : 1.0);
+        walk += n * probes * (group.slots_smem ? (group.isolate ? 350.0 : 500.0) : 3500.0) / std::max(1u, group.ns);
+        latency = std::max(latency, probes * (group.slots_smem ? 300.0 : 2500.0) + 60.0 * build);
+    }
+    const double per_sm = trials / sms;
+    uint32_t warps = force_lanes > 0 ? uint32_t(force_lanes) : 0;
+    if (!warps) {
+        double best = 1e300;
+        for (uint32_t w = 1; w <= kMaxLaneWarps; ++w) {
+            const double lanes = w * std::min(32.0, std::ceil(per_sm / w));
+            const double step = (8000.0 + 740.0 * w) * (wide_domain ? 1.15 : 1.0);
+            // trials of even length run in whole waves; the more their lengths
+            // differ, the less the last wave waits for
+            const double waves = per_sm / lanes;
+            const double even = std::max(0.0, 1.0 - 3.0 * spread / trials * std::sqrt(waves));
+            const double tail = even * (std::ceil(waves) - waves) + (1.0 - even) * 0.5 + 0.1;
+            const double cycles = waves <= 1.0 ? longest * step : passes / trials * step * (waves + tail);
+            const double total = cycles + 4000.0 * per_sm / lanes + 30000.0;
+            if (total < best) {
+                best = total;
+                warps = w;
+            }
+        }
+        const double group_cycles = std::max(produce, walk) / trials * std::ceil(per_sm) + 0.6 * latency + 24000.0;
+        if (best >= 0.9 * group_cycles) return lp;
+    }
+    lp.variant = group.variant;
+    lp.ctas = sms;
+    lp.share = uint32_t(std::min(32.0, std::max(1.0, std::ceil(per_sm / warps))));
+    lp.region_bytes = (uint64_t(max_b) * (group.variant == 0 ? 8 : 16) + 127) / 128 * 128;
+    lp.smem_bytes = kLaneTableBytes + warps * kLaneFoldBytes;
+    lp.regions_bytes = lp.region_bytes * sms * warps * lp.share;
+    lp.stock_bytes = uint64_t(sms) * warps * kLaneStockBytes;
+    // tables of all lanes: 13.0 GB at B = 24576; never more than an eighth of the device
+    if (lp.regions_bytes + lp.stock_bytes > memory_bytes / 8 || lp.smem_bytes > smem_optin) return lp;
+    lp.warps = warps;
+    return lp;
+}
+
 // Queue the engine launches over `jobs` (already on the device in d_jobs) --
 // one per plan class, class c covering the job-table range
 // [bounds[c], bounds[c + 1]) and so a contiguous range of global trial
@@ -314,6 +422,7 @@ int Ctx::run(const std::vector<Job>& jobs, uint64_t total, cudaStream_t st, uint
     const uint32_t nclass = uint32_t(bounds.size()) - 1;
     if (nclass < 1 || nclass > kMaxClasses) return fail(CMC_EINVAL, "bad plan classes");
     std::vector<Plan> plans(nclass);
+    std::vector<LanePlan> lanes(nclass);
     std::vector<double> class_work(nclass, 0.0), class_trials(nclass, 0.0);
     uint32_t heaviest = 0;
     uint64_t heaviest_trials = 0;
@@ -334,7 +443,8 @@ int Ctx::run(const std::vector<Job>& jobs, uint64_t total, cudaStream_t st, uint
             heaviest_trials = trials;
             heaviest = c;
         }
-        text += (c ? " | " : "") + plan_text;
+        lanes[c] = plan_lanes(part, plans[c]);
+        text += (c ? " | " : "") + plan_text + lanes_text(lanes[c]);
     }
     // Several classes run as ONE persistent launch unless disabled or a class
     // uses the split engine; the classes then run side by side, so each gets
@@ -344,7 +454,9 @@ int Ctx::run(const std::vector<Job>& jobs, uint64_t total, cudaStream_t st, uint
     std::vector<uint64_t> region(nclass, 0);
     uint64_t pool = 0;
     for (uint32_t c = 0; c < nclass; ++c) {
-        const uint64_t need = (plans[c].gslot_bytes + 255) / 256 * 256 + (plans[c].gcache_bytes + 255) / 256 * 256;
+        const uint64_t need = lanes[c].warps
+                                  ? lanes[c].regions_bytes + lanes[c].stock_bytes
+                                  : (plans[c].gslot_bytes + 255) / 256 * 256 + (plans[c].gcache_bytes + 255) / 256 * 256;
         if (fuse) {
             region[c] = pool;
             pool += need;
@@ -357,7 +469,16 @@ int Ctx::run(const std::vector<Job>& jobs, uint64_t total, cudaStream_t st, uint
     int rc = grow(d_bits, bits_cap, words, "failure bitmap");
     if (rc) return rc;
     // walk slots, then the groups' round caches, per pool region
-    if (pool && (rc = grow(d_slots, slots_cap, size_t(pool), "slot and cache pool"))) return rc;
+    if (pool && (rc = grow(d_slots, slots_cap, size_t(pool), "slot and cache pool"))) {
+        const bool any_lanes = std::any_of(lanes.begin(), lanes.end(), [](const LanePlan& l) { return l.warps; });
+        if (rc != CMC_ENOMEM || !any_lanes || force_lanes > 0) return rc;
+        // no room for the lanes' tables: the group engine needs less
+        const int kept = force_lanes;
+        force_lanes = 0;
+        rc = run(jobs, total, st, value_base, d_out, d_count, out_cap_now, job_failed, job_done, bounds_in);
+        force_lanes = kept;
+        return rc;
+    }
     if ((rc = cuda(cudaMemsetAsync(d_ctrl, 0, nclass * sizeof(Ctrl), st), "memset ctrl"))) return rc;
     if ((rc = cuda(cudaMemsetAsync(d_bits, 0, words * 4, st), "memset bitmap"))) return rc;
     // timing events stay out of captured graphs: a replay records them
@@ -410,10 +531,10 @@ int Ctx::run(const std::vector<Job>& jobs, uint64_t total, cudaStream_t st, uint
     std::vector<bool> launched(nclass, false);
     // Classes with pooled direct passes run their own kernel, unfused.
     for (uint32_t lead = 0; lead < nclass && fuse; ++lead) {
-        if (launched[lead] || plans[lead].pool_stage) continue;
+        if (launched[lead] || plans[lead].pool_stage || lanes[lead].warps) continue;
         std::vector<uint32_t> members;
         for (uint32_t c = lead; c < nclass; ++c)
-            if (!launched[c] && !plans[c].pool_stage && plans[c].variant == plans[lead].variant &&
+            if (!launched[c] && !plans[c].pool_stage && !lanes[c].warps && plans[c].variant == plans[lead].variant &&
                 plans[c].slots_smem == plans[lead].slots_smem)
                 members.push_back(c);
         if (members.size() < 2) continue;
@@ -441,6 +562,31 @@ int Ctx::run(const std::vector<Job>& jobs, uint64_t total, cudaStream_t st, uint
     for (uint32_t c = 0; c < nclass; ++c) {
         if (launched[c]) continue;
         const Plan& pl = plans[c];
+        if (lanes[c].warps) {
+            const LanePlan& lp = lanes[c];
+            const EngineArgs e = class_args(c);
+            LaneArgs a{};
+            a.jobs = e.jobs;
+            a.njobs = e.njobs;
+            a.total = e.total;
+            a.gidx_begin = e.gidx_begin;
+            a.ctrl = e.ctrl;
+            a.fail_bits = e.fail_bits;
+            a.job_failed = e.job_failed;
+            a.t0 = e.t0;
+            a.regions = d_slots + region[c];
+            a.region_bytes = lp.region_bytes;
+            a.hops = kLaneHops;
+            a.stock = reinterpret_cast<uint32_t*>(a.regions + lp.regions_bytes);
+            a.share = lp.share;
+            void* args[] = {&a};
+            if ((rc = cuda(cudaLaunchKernel(lane_kernel(lp.variant), dim3(lp.ctas), dim3(lp.warps * 32), args,
+                                            lp.smem_bytes, st),
+                           "lane engine launch")))
+                return rc;
+            ++kernels;
+            continue;
+        }
         if (pl.walker_ctas) {
             if ((rc = grow(d_ghdr, ghdr_cap, pl.ns, "slot headers"))) return rc;
             if ((rc = cuda(cudaMemsetAsync(d_ghdr, 0, size_t(pl.ns) * sizeof(GSlotHeader), st), "memset slots")))
@@ -524,6 +670,12 @@ const void* fused_engine_kernel(int variant, bool smem_slots) {
                           : (const void*)cmc_engine_fused<uint32_t, uint32_t, true, false>;
 }
 
+const void* lane_kernel(int variant) {
+    return variant == 0   ? (const void*)cmc_lanes<true, false>
+           : variant == 1 ? (const void*)cmc_lanes<false, false>
+                          : (const void*)cmc_lanes<false, true>;
+}
+
 // Every engine kernel may use up to the device's opt-in shared memory.  Set
 // once per device and never lowered, so launches of different plans -- and
 // graphs captured from them -- are valid whatever ran in between.
@@ -536,7 +688,8 @@ int engine_smem_cap(size_t optin) {
                          fused_engine_kernel(0, true), fused_engine_kernel(1, true),
                          fused_engine_kernel(2, true), fused_engine_kernel(0, false),
                          fused_engine_kernel(1, false), fused_engine_kernel(2, false),
-                         engine_kernel(0, true, true), engine_kernel(1, true, true)};
+                         engine_kernel(0, true, true), engine_kernel(1, true, true),
+                         lane_kernel(0), lane_kernel(1), lane_kernel(2)};
     for (const void* fn : fns)
         if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(optin)) != cudaSuccess)
             return CMC_ECUDA;
@@ -554,6 +707,7 @@ int Ctx::init(int dev) {
                     prop.major, prop.minor);
     sms = prop.multiProcessorCount;
     smem_optin = prop.sharedMemPerBlockOptin;
+    memory_bytes = prop.totalGlobalMem;
     if (engine_smem_cap(smem_optin)) {
         cudaGetLastError();
         return fail(CMC_ECUDA, "cudaFuncSetAttribute on the engine kernels failed");
@@ -707,7 +861,7 @@ std::string Ctx::graph_key(const std::vector<Job>& jobs, const std::vector<uint3
     snprintf(b, sizeof b, "|%llu|%llu|%u/%u/%u/%u/%u/%d/%d/%d/%u/%u/%d|%p/%p/%p/%p/%p/%p/%p/%p",
              (unsigned long long)total, (unsigned long long)dev_cap, force_wg, force_ng,
              force_global_slots, force_walkers, max_slots_per_group, force_walker_ctas, force_isolate,
-             force_method, spin_limit, map_chains * 16 + fill_blocks, use_fused, (void*)d_jobs, (void*)d_bits, (void*)d_out, (void*)d_slots,
+             force_method, spin_limit, map_chains * 16 + fill_blocks, use_fused + 2 * force_lanes + 2 * 64 * force_pool, (void*)d_jobs, (void*)d_bits, (void*)d_out, (void*)d_slots,
              (void*)d_ctrl, (void*)d_job_failed, (void*)h_failed, (void*)h_nf);
     return key + b;
 }
@@ -1073,6 +1227,7 @@ int cmc_set_option(cmc_ctx* ctx, const char* name, int64_t value) {
     else if (n == "groups" && value >= 0 && value <= cmc::kMaxGroups) c->force_ng = uint32_t(value);
     else if (n == "global_slots" && (value == 0 || value == 1)) c->force_global_slots = uint32_t(value);
     else if (n == "method" && value >= -1 && value <= 2) c->force_method = int(value);
+    else if (n == "lanes" && value >= -1 && value <= int64_t(cmc::kMaxLaneWarps)) c->force_lanes = int(value);
     else if (n == "pool" && value >= -1 && value <= 1) c->force_pool = int(value);
     else if (n == "graph" && (value == 0 || value == 1)) c->use_graphs = int(value);
     else if (n == "fused" && (value == 0 || value == 1)) c->use_fused = int(value);
@@ -1141,6 +1296,7 @@ int cmc_plan_describe(const cmc_params* params, uint32_t count, uint32_t sms, ui
     int rc = c.make_job(*params, 0, count, 0, jobs[0]);
     cmc::Plan pl;
     if (!rc) rc = c.plan(jobs, pl);
+    if (!rc) c.plan_text += cmc::lanes_text(c.plan_lanes(jobs, pl));
     snprintf(out, cap, "%s", (rc ? c.err : c.plan_text).c_str());
     if (rc) cmc::set_thread_error(c.err);
     return rc;

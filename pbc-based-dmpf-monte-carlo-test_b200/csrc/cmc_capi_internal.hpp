@@ -30,6 +30,16 @@ struct Plan {
     uint32_t pool_fold = 0;       // pooled direct passes: bytes per fold table (0: unfolded)
 };
 
+// How a launch runs in the lane engine (cmc_lanes.cu).
+struct LanePlan {
+    uint32_t warps = 0;         // per CTA (0: the group engine runs the launch)
+    uint32_t share = 32;        // lanes per warp that take trials
+    uint32_t ctas = 0, smem_bytes = 0;
+    int variant = 0;            // as Plan::variant
+    uint64_t region_bytes = 0;  // per lane
+    uint64_t regions_bytes = 0, stock_bytes = 0;
+};
+
 uint32_t choose_method(uint32_t h, uint64_t domain, double candidates, int force, bool may_allocate);
 // Raises the engine kernels' dynamic shared-memory limit to the device's opt-in maximum.
 int engine_smem_cap(size_t optin);
@@ -37,6 +47,7 @@ int engine_smem_cap(size_t optin);
 // placement, and the fused kernel of the same kind.
 const void* engine_kernel(int variant, bool smem_slots, bool pooled = false);
 const void* fused_engine_kernel(int variant, bool smem_slots);
+const void* lane_kernel(int variant);
 // Estimated cost of one trial in AES-block equivalents (seeds, map, 0.1 t for the walk).
 double job_cost(const Job& j);
 
@@ -51,6 +62,7 @@ struct Ctx {
     int device = -1;
     int sms = 0;
     size_t smem_optin = 0;
+    uint64_t memory_bytes = 180ull << 30;  // device memory (the planner's default: B200)
     cudaStream_t stream = nullptr;       // the context's own stream
     cudaStream_t user_stream = nullptr;  // cmc_set_stream override
     cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
@@ -99,6 +111,7 @@ struct Ctx {
     uint32_t* h_nf = nullptr;                // pinned failure count of the last batched call
     std::string graph_state;                 // "eager", "captured" or "replayed"
     int force_method = -1;  // -1 auto, 0 direct, 1 cache (shared if h <= 12, else global), 2 global cache
+    int force_lanes = -1;   // lane engine: -1 auto, 0 off, N warps per CTA
     int force_pool = -1;    // pooled direct passes: -1 auto, 0 off, 1 on where they apply
     bool plan_no_dfold = false;  // plan() re-run without room for direct passes' fold tables
     bool may_allocate = true;  // false: no global round cache, global slots only if unavoidable
@@ -114,6 +127,7 @@ struct Ctx {
     int grow(T*& ptr, size_t& cap, size_t need, const char* what);
     int make_job(const cmc_params& p, uint32_t first, uint32_t count, uint64_t base, Job& j);
     int plan(const std::vector<Job>& jobs, Plan& pl);
+    LanePlan plan_lanes(const std::vector<Job>& jobs, const Plan& group) const;
     int upload_jobs(const std::vector<Job>& jobs, cudaStream_t st);
     int run(const std::vector<Job>& jobs, uint64_t total, cudaStream_t st, uint32_t value_base,
             uint32_t* d_out, uint32_t* d_count, uint64_t out_cap, unsigned long long* job_failed,
