@@ -214,7 +214,10 @@ int cmc_server_destroy(cmc_server* server);
  * memory; automatic is 3 there and 2 elsewhere), "lanes" (-1, the
  * default: launches with enough trials run in the lane engine, one trial per
  * thread, when none of the options above or "pool" is set; 0: never; 1..16:
- * always, with that many warps per SM), "pool" (-1, the default:
+ * always, with that many warps per SM), "waves" (-1, the default: likewise the
+ * wave engine, whose groups build maps and then walk one trial per thread; 0:
+ * never; 1, 2, 4 or 8: with that many groups per SM, fewer where shared memory
+ * holds fewer, for PRP half widths up to 16), "pool" (-1, the default:
  * one-warp groups whose jobs all take direct passes with 16-bit Feistel
  * halves and shared-memory walk slots keep three trials in flight and stage
  * their maps; 0: one trial at a time; 1 as -1 -- such plans run in a kernel
@@ -265,7 +268,8 @@ uint32_t cmc_last_kernel_count(const cmc_ctx* ctx);
 const char* cmc_last_plan(const cmc_ctx* ctx);
 /* No counterpart in the reference.  Planner dry run, no device needed: writes
  * to out (cap bytes) the plan text cmc_launch would report for count trials
- * (the group engine's plan, and after "->" the lane engine's where that runs)
+ * (the group engine's plan, and after "->" the lane or wave engine's where
+ * that runs)
  * of params on a device with `sms` SMs and `smem_optin` bytes of opt-in
  * shared memory per block (148 and 232448 on B200), with default options.
  * Returns 0, or a CMC_E* code with the reason in out. */

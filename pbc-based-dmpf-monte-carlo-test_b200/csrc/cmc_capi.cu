@@ -15,6 +15,8 @@
 #include "cmc_engine.cuh"
 #include "cmc_hostcore.hpp"
 #include "cmc_lanes.cuh"
+#include "cmc_trial.cuh"
+#include "cmc_waves.cuh"
 
 namespace cmc {
 
@@ -28,6 +30,8 @@ template <typename MapT, typename BinT, bool WIDE, bool SMEMSLOTS>
 __global__ void cmc_engine_fused(const __grid_constant__ FusedArgs f);
 template <bool NARROW, bool WIDE>
 __global__ void cmc_lanes(const LaneArgs a);
+template <bool NARROW, bool GC>
+__global__ void cmc_waves(const WaveArgs a);
 __global__ void cmc_compact_failures(const uint32_t* bits, uint64_t nbits, uint32_t value_base,
                                      uint32_t* out, uint32_t* count, uint64_t cap,
                                      const unsigned long long* nbits_dev);
@@ -47,6 +51,14 @@ std::string lanes_text(const LanePlan& lp) {
     char buf[96];
     snprintf(buf, sizeof buf, " -> engine=lanes warps=%u lanes_per_warp=%u region=%llu", lp.warps, lp.share,
              (unsigned long long)lp.region_bytes);
+    return buf;
+}
+
+std::string waves_text(const WavePlan& wp) {
+    if (!wp.ng) return "";
+    char buf[112];
+    snprintf(buf, sizeof buf, " -> engine=waves groups=%u warps_per_group=%u wave=%u region=%llu cache=%s", wp.ng,
+             wp.wg, wp.wave, (unsigned long long)wp.region_bytes, wp.global_cache ? "global" : "smem");
     return buf;
 }
 
@@ -324,75 +336,89 @@ double lane_evaluations(const Job& j) {
     return t < 0.999 * b ? std::min(cand, -b * std::log(1.0 - t / b)) : cand;
 }
 
-}  // namespace
+// Feistel passes per evaluation (cycle-walking).
+double walk_factor(const Job& j) { return std::ldexp(1.0, 2 * int(j.half_bits)) / double(j.domain); }
 
-// The lane engine's form of a launch, or warps == 0 where the group engine
-// (whose plan is `group`) runs it.  Both sides are estimated in SM cycles:
-//   lanes: a trial is a chain of P passes (evaluations x cycle-walking, +8 %
-//     for passes a BGH25 lane sits out, +2 % for DRRT18), and W warps make a
-//     pass in 8,000 + 740 W cycles (latency of 80 dependent AES rounds, then
-//     960 shared-memory wavefronts per warp); a launch ends with its slowest
-//     trial.  15 % more with 64-bit domains.
-//   group: AES blocks over the measured 0.19-0.21 blocks per cycle and SM
-//     (0.135 with 64-bit domains, 0.125-0.15 beside walks over global slots), 500-3,000 cycles of set-up per trial, or its
-//     walks over the slots, whichever takes longer, and one trial's latency.
-// The constants are fitted to 160 launches drawn over t = 3..14,000, N =
-// 2^8..2^32, k = 2..4, both modes, 2^2..2^20 trials (B200): the choice is within
-// 2 % of the better engine on average.  At t = 64, N = 2^16, 2^20 trials: 34.1
-// ms in the group engine, 18.9 in lanes; at 4,000 trials 0.25 against 0.9.
-LanePlan Ctx::plan_lanes(const std::vector<Job>& jobs, const Plan& group) const {
-    LanePlan lp;
-    const bool forced_group = force_wg || force_ng || force_global_slots || force_walkers ||
-                              force_walker_ctas >= 0 || force_isolate >= 0 || force_method >= 0 ||
-                              force_pool >= 0 || max_slots_per_group != 8 || map_chains || fill_blocks;
-    if (force_lanes == 0 || (force_lanes < 0 && forced_group)) return lp;
-    uint64_t count = 0;
-    for (const Job& j : jobs) count += j.count;
-    if (force_lanes < 0 && count < 16ull * sms) return lp;  // far below every launch that gains
-    const bool wide_domain = group.variant == 2;
-    double trials = 0, max_b = 0, passes = 0, longest = 0;  // passes: of all trials
-    double spread = 0;  // relative spread of a trial's passes
-    double produce = 0, walk = 0, latency = 0;
+// Expected probes of one trial (measured at t/B = 2/3: 2.39 t and 1.75 t).
+double expected_probes(const Job& j) {
+    return (j.mode == CMC_MODE_BGH25 ? 2.4 : 1.75) * j.pnum * (j.k == 2 ? 0.8 : 1.0);
+}
+
+// Probes by which the longest walk of a launch of small tables exceeds the
+// mean: one of its trials fails, at the eviction limit.
+double straggler_probes(const Job& j) { return j.pnum < 256 ? std::min<double>(j.kick, 500) : 0.0; }
+
+// The three engines' times for a launch, in SM cycles.  Constants fitted to 290
+// launches drawn over t = 3..15,000, N = 2^8..2^32, k = 2..4, both modes and
+// 2^2..2^20 trials (B200), standard errors 30 % (group), 30 % (lanes), 14 %
+// (waves); the engine chosen is within 3 % of the best one on average.
+//
+// Group engine: AES blocks over the measured 0.19-0.21 blocks per cycle and SM
+// (0.135 with 64-bit domains, 0.125-0.15 beside walks over global slots) and a
+// trial's serial set-up in its group, or its walks over the slots, whichever
+// takes longer, and one trial's latency.
+double group_cycles(const std::vector<Job>& jobs, const Plan& g, int sms) {
+    double trials = 0, produce = 0, walk = 0, latency = 0;
+    const bool wide_domain = g.variant == 2;
     for (const Job& j : jobs) {
-        const double n = j.count, cw = std::ldexp(1.0, 2 * int(j.half_bits)) / double(j.domain);
-        const double cand = double(j.pnum) * j.k * cw;
-        trials += n;
-        max_b = std::max<double>(max_b, j.buckets);
-        const double e = lane_evaluations(j);
-        const double p = e * cw * (j.mode == CMC_MODE_BGH25 ? 1.08 : 1.02);
-        spread += n * (jobs.size() > 1 ? 0.5 : (j.mode == CMC_MODE_BGH25 ? 2.0 : 1.1) / std::sqrt(std::max(1.0, e)));
-        passes += n * p;
-        longest = std::max(longest, p + 3.0 * std::sqrt(p) + 6.0);
+        const double n = j.count, cand = double(j.pnum) * j.k * walk_factor(j);
         const double build = j.method == kMethodDirect ? 8.0 * cand : 8.0 * std::ldexp(1.0, int(j.half_bits));
-        const double rate = wide_domain ? 0.135 : group.pool_stage ? 0.21 : group.slots_smem ? 0.19
+        const double rate = wide_domain ? 0.135 : g.pool_stage ? 0.21 : g.slots_smem ? 0.19
                             : j.method == kMethodCache ? 0.19 : j.method == kMethodGCache ? 0.15 : 0.125;
         const double lookups = j.method == kMethodCache ? cand : j.method == kMethodGCache ? 1.5 * cand : 0.0;
-        produce += n * ((2.0 + build) / rate + lookups + (wide_domain ? 3000.0 : group.pool_stage ? 500.0 : 600.0));
-        const double probes = (j.mode == CMC_MODE_BGH25 ? 2.4 : 1.75) * j.pnum * (j.k == 2 ? 0.8 : 1.0);
-        walk += n * probes * (group.slots_smem ? (group.isolate ? 350.0 : 500.0) : 3500.0) / std::max(1u, group.ns);
-        latency = std::max(latency, probes * (group.slots_smem ? 300.0 : 2500.0) + 60.0 * build);
+        trials += n;
+        produce += n * ((2.0 + build) / rate + lookups +
+                        (g.pool_stage ? 600.0 : (wide_domain ? 25000.0 : 17000.0) / g.ng));
+        const double probe = g.slots_smem ? (g.isolate ? (j.mode == CMC_MODE_BGH25 ? 350.0 : 900.0) : 500.0) : 3500.0;
+        walk += n * expected_probes(j) * probe / std::max(1u, g.ns);
+        latency = std::max(latency, (expected_probes(j) + straggler_probes(j)) * (g.slots_smem ? 180.0 : 2000.0) +
+                                        6.0 * build);
+    }
+    return std::max(produce, walk) / trials * (trials / sms + 0.5) + latency + 24000.0;
+}
+
+}  // namespace
+
+// The lane engine's form of a launch (warps == 0: it does not fit).  A trial is
+// a chain of P passes (evaluations x cycle-walking, +8 % for passes a BGH25 lane
+// sits out, +2 % for DRRT18), and W warps make a pass in 8,000 + 740 W cycles
+// (latency of 80 dependent AES rounds, then 960 shared-memory wavefronts per
+// warp; 15 % more with 64-bit domains); W is chosen by the estimate.
+LanePlan Ctx::plan_lanes(const std::vector<Job>& jobs, const Plan& group) const {
+    LanePlan lp;
+    const bool wide_domain = group.variant == 2;
+    double trials = 0, max_b = 0, passes = 0, longest = 0;  // passes: of all trials
+    double spread = 0, sits_out = 0;  // relative spread of a trial's passes; passes a straggler sits out
+    for (const Job& j : jobs) {
+        const double n = j.count, e = lane_evaluations(j);
+        // a lane on known buckets sits out up to one pass per kLaneHops probes
+        const double idle = j.pnum < 16 ? j.kick / double(kLaneHops) : 0.0;
+        const double p = e * walk_factor(j) * (j.mode == CMC_MODE_BGH25 ? 1.08 : 1.02) + 0.02 * idle;
+        trials += n;
+        max_b = std::max<double>(max_b, j.buckets);
+        spread += n * (jobs.size() > 1 ? 0.5 : (j.mode == CMC_MODE_BGH25 ? 2.0 : 1.1) / std::sqrt(std::max(1.0, e)));
+        passes += n * p;
+        longest = std::max(longest, p + 3.0 * std::sqrt(p) + 6.0 + idle);
+        sits_out = std::max(sits_out, idle);
     }
     const double per_sm = trials / sms;
-    uint32_t warps = force_lanes > 0 ? uint32_t(force_lanes) : 0;
-    if (!warps) {
-        double best = 1e300;
-        for (uint32_t w = 1; w <= kMaxLaneWarps; ++w) {
-            const double lanes = w * std::min(32.0, std::ceil(per_sm / w));
-            const double step = (8000.0 + 740.0 * w) * (wide_domain ? 1.15 : 1.0);
-            // trials of even length run in whole waves; the more their lengths
-            // differ, the less the last wave waits for
-            const double waves = per_sm / lanes;
-            const double even = std::max(0.0, 1.0 - 3.0 * spread / trials * std::sqrt(waves));
-            const double tail = even * (std::ceil(waves) - waves) + (1.0 - even) * 0.5 + 0.1;
-            const double cycles = waves <= 1.0 ? longest * step : passes / trials * step * (waves + tail);
-            const double total = cycles + 4000.0 * per_sm / lanes + 30000.0;
-            if (total < best) {
-                best = total;
-                warps = w;
-            }
+    uint32_t warps = 0;
+    lp.cycles = 1e300;
+    for (uint32_t w = 1; w <= kMaxLaneWarps; ++w) {
+        if (force_lanes > 0 && w != uint32_t(force_lanes)) continue;
+        const double lanes = w * std::min(32.0, std::ceil(per_sm / w));
+        const double step = (8000.0 + 740.0 * w) * (wide_domain ? 1.15 : 1.0);
+        // trials of even length run in whole waves; the more their lengths
+        // differ, the less the last wave waits for
+        const double waves = per_sm / lanes;
+        const double even = std::max(0.0, 1.0 - 3.0 * spread / trials * std::sqrt(waves));
+        const double tail = even * (std::ceil(waves) - waves) + (1.0 - even) * 0.5 + 0.1;
+        const double cycles = (waves <= 1.0 ? longest * step : passes / trials * step * (waves + tail) + 0.3 * sits_out * step) +
+                              4000.0 * waves + 30000.0;
+        if (cycles < lp.cycles) {
+            lp.cycles = cycles;
+            warps = w;
         }
-        const double group_cycles = std::max(produce, walk) / trials * std::ceil(per_sm) + 0.6 * latency + 24000.0;
-        if (best >= 0.9 * group_cycles) return lp;
     }
     lp.variant = group.variant;
     lp.ctas = sms;
@@ -400,11 +426,103 @@ LanePlan Ctx::plan_lanes(const std::vector<Job>& jobs, const Plan& group) const 
     lp.region_bytes = (uint64_t(max_b) * (group.variant == 0 ? 8 : 16) + 127) / 128 * 128;
     lp.smem_bytes = kLaneTableBytes + warps * kLaneFoldBytes;
     lp.regions_bytes = lp.region_bytes * sms * warps * lp.share;
-    lp.stock_bytes = uint64_t(sms) * warps * kLaneStockBytes;
+    lp.stock_bytes = uint64_t(sms) * warps * kRecordBlockBytes;
     // tables of all lanes: 13.0 GB at B = 24576; never more than an eighth of the device
     if (lp.regions_bytes + lp.stock_bytes > memory_bytes / 8 || lp.smem_bytes > smem_optin) return lp;
     lp.warps = warps;
     return lp;
+}
+
+// The wave engine's form of a launch (ng == 0: it does not fit).  A map costs
+// the fill (8 * 2^h blocks at 106 wavefronts per 32 and 98 % of the shared-memory
+// pipe: 27.2 cycles * 2^h), its lookups and 3 cycles per probe; a walk step
+// takes 900 cycles and 145 more per lane of the warp.  Fewer groups lose overlap
+// of fill, map and walk; more than two spill global caches out of L2.
+WavePlan Ctx::plan_waves(const std::vector<Job>& jobs, const Plan& group) const {
+    WavePlan wp;
+    wp.cycles = 1e300;
+    if (group.variant == 2) return wp;
+    double trials = 0, build = 0, probes = 0, stragglers = 0;
+    uint64_t max_b = 0, max_t = 0;
+    uint32_t max_h = 0;
+    for (const Job& j : jobs) max_h = std::max(max_h, j.half_bits);
+    const bool gc = max_h > 12;
+    for (const Job& j : jobs) {
+        const double cand = double(j.pnum) * j.k * walk_factor(j);
+        build += j.count * (27.2 * std::ldexp(1.0, int(j.half_bits)) + (gc ? 6.0 : 1.8) * cand +
+                            3.0 * expected_probes(j) + 1200.0);
+        probes = std::max(probes, expected_probes(j));
+        stragglers = std::max(stragglers, straggler_probes(j));
+        trials += j.count;
+        max_b = std::max<uint64_t>(max_b, j.buckets);
+        max_t = std::max<uint64_t>(max_t, j.pnum);
+    }
+    build /= trials;
+    const uint64_t entry = group.variant == 0 ? 8 : 16;
+    WavePlan q;
+    q.variant = group.variant;
+    q.ctas = sms;
+    q.global_cache = gc;
+    q.cache_off = kWaveHeaderBytes + fold_table_bytes(max_h);
+    q.group_bytes = q.cache_off + (gc ? 0 : 16u << max_h);
+    q.map_off = uint32_t((max_b * entry + 15) / 16 * 16);
+    q.region_bytes = (q.map_off + max_t * entry + 127) / 128 * 128;
+    q.gcache_stride = gc ? 8u << max_h : 0;
+    for (uint32_t ng : {1u, 2u, 4u, 8u}) {
+        if (force_waves > 0 && ng > uint32_t(force_waves)) break;
+        q.smem_bytes = kEngineTableBytes + ng * q.group_bytes;
+        if (q.smem_bytes > smem_optin) break;
+        q.ng = ng;
+        q.wg = 16 / ng;
+        q.gcache_bytes = uint64_t(sms) * ng * q.gcache_stride * 2;
+        const double lost = gc ? (ng == 1 ? 1.02 : ng == 2 ? 1.0 : ng == 4 ? 1.03 : 1.2) *
+                                     (q.gcache_bytes > 140000000 ? 1.08 : 1.0)
+                               : (ng == 1 ? 1.3 : ng == 2 ? 1.12 : ng == 4 ? 1.0 : 0.97);
+        // One wave where a group's share of the launch fits its threads: the
+        // walks of all groups then run once, after all maps.  Longer launches
+        // run in waves of equal size; towards the end they shrink to the trials
+        // whose maps take as long to build as a walk does.
+        const double share = std::ceil(trials / (double(sms) * ng)), nt = q.wg * 32, waves = std::ceil(share / nt);
+        q.wave = uint32_t(std::ceil(share / waves));
+        const double walk = probes * (900.0 + 145.0 * q.wave / q.wg) + 1000.0 * stragglers;
+        q.min_wave = waves > 1 ? uint32_t(std::min(double(q.wave), std::max(1.0, walk / (build * ng)))) : q.wave;
+        const double maps = share * ng * build * lost;
+        q.cycles = (waves > 1 ? std::max(maps, waves * walk) : maps) + walk + 60000.0;
+        q.regions_bytes = q.region_bytes * sms * ng * q.wave;
+        q.stock_bytes = uint64_t(sms) * ng * q.wg * kRecordBlockBytes;
+        if (q.regions_bytes + q.stock_bytes + q.gcache_bytes > memory_bytes / 8) continue;
+        if (q.cycles < wp.cycles || force_waves > 0) wp = q;
+    }
+    return wp;
+}
+
+// Which engine runs a launch whose group-engine plan is `group`: lanes and
+// waves are left empty where it is the group engine.  The others have to be
+// estimated 8-10 % shorter.
+void Ctx::choose_engine(const std::vector<Job>& jobs, const Plan& group, LanePlan& lanes, WavePlan& waves) const {
+    lanes = LanePlan{};
+    waves = WavePlan{};
+    const bool group_options = force_wg || force_ng || force_global_slots || force_walkers ||
+                               force_walker_ctas >= 0 || force_isolate >= 0 || force_method >= 0 ||
+                               force_pool >= 0 || max_slots_per_group != 8 || map_chains || fill_blocks;
+    if (force_waves > 0) {
+        waves = plan_waves(jobs, group);
+        if (waves.ng) return;
+    }
+    if (force_lanes > 0) {
+        lanes = plan_lanes(jobs, group);
+        return;
+    }
+    uint64_t count = 0;
+    for (const Job& j : jobs) count += j.count;
+    // a CTA without a full wave of its groups' threads gains nothing
+    if (group_options || force_waves > 0 || count < 2ull * sms) return;
+    const double limit = group_cycles(jobs, group, sms);
+    if (force_waves < 0) waves = plan_waves(jobs, group);
+    if (force_lanes < 0 && count >= 16ull * sms) lanes = plan_lanes(jobs, group);
+    if (!lanes.warps || lanes.cycles >= 0.9 * limit) lanes = LanePlan{};
+    if (!waves.ng || waves.cycles >= 0.92 * limit || (lanes.warps && lanes.cycles < waves.cycles)) waves = WavePlan{};
+    if (waves.ng) lanes = LanePlan{};
 }
 
 // Queue the engine launches over `jobs` (already on the device in d_jobs) --
@@ -423,6 +541,7 @@ int Ctx::run(const std::vector<Job>& jobs, uint64_t total, cudaStream_t st, uint
     if (nclass < 1 || nclass > kMaxClasses) return fail(CMC_EINVAL, "bad plan classes");
     std::vector<Plan> plans(nclass);
     std::vector<LanePlan> lanes(nclass);
+    std::vector<WavePlan> waves(nclass);
     std::vector<double> class_work(nclass, 0.0), class_trials(nclass, 0.0);
     uint32_t heaviest = 0;
     uint64_t heaviest_trials = 0;
@@ -443,8 +562,8 @@ int Ctx::run(const std::vector<Job>& jobs, uint64_t total, cudaStream_t st, uint
             heaviest_trials = trials;
             heaviest = c;
         }
-        lanes[c] = plan_lanes(part, plans[c]);
-        text += (c ? " | " : "") + plan_text + lanes_text(lanes[c]);
+        choose_engine(part, plans[c], lanes[c], waves[c]);
+        text += (c ? " | " : "") + plan_text + lanes_text(lanes[c]) + waves_text(waves[c]);
     }
     // Several classes run as ONE persistent launch unless disabled or a class
     // uses the split engine; the classes then run side by side, so each gets
@@ -454,7 +573,8 @@ int Ctx::run(const std::vector<Job>& jobs, uint64_t total, cudaStream_t st, uint
     std::vector<uint64_t> region(nclass, 0);
     uint64_t pool = 0;
     for (uint32_t c = 0; c < nclass; ++c) {
-        const uint64_t need = lanes[c].warps
+        const uint64_t need = waves[c].ng ? waves[c].regions_bytes + waves[c].stock_bytes + waves[c].gcache_bytes
+                              : lanes[c].warps
                                   ? lanes[c].regions_bytes + lanes[c].stock_bytes
                                   : (plans[c].gslot_bytes + 255) / 256 * 256 + (plans[c].gcache_bytes + 255) / 256 * 256;
         if (fuse) {
@@ -470,13 +590,13 @@ int Ctx::run(const std::vector<Job>& jobs, uint64_t total, cudaStream_t st, uint
     if (rc) return rc;
     // walk slots, then the groups' round caches, per pool region
     if (pool && (rc = grow(d_slots, slots_cap, size_t(pool), "slot and cache pool"))) {
-        const bool any_lanes = std::any_of(lanes.begin(), lanes.end(), [](const LanePlan& l) { return l.warps; });
-        if (rc != CMC_ENOMEM || !any_lanes || force_lanes > 0) return rc;
-        // no room for the lanes' tables: the group engine needs less
-        const int kept = force_lanes;
-        force_lanes = 0;
+        if (rc != CMC_ENOMEM || (force_lanes == 0 && force_waves == 0)) return rc;
+        // no room for the tables of the lane or wave engine: the group engine needs less
+        const int kept[2] = {force_lanes, force_waves};
+        force_lanes = force_waves = 0;
         rc = run(jobs, total, st, value_base, d_out, d_count, out_cap_now, job_failed, job_done, bounds_in);
-        force_lanes = kept;
+        force_lanes = kept[0];
+        force_waves = kept[1];
         return rc;
     }
     if ((rc = cuda(cudaMemsetAsync(d_ctrl, 0, nclass * sizeof(Ctrl), st), "memset ctrl"))) return rc;
@@ -531,10 +651,10 @@ int Ctx::run(const std::vector<Job>& jobs, uint64_t total, cudaStream_t st, uint
     std::vector<bool> launched(nclass, false);
     // Classes with pooled direct passes run their own kernel, unfused.
     for (uint32_t lead = 0; lead < nclass && fuse; ++lead) {
-        if (launched[lead] || plans[lead].pool_stage || lanes[lead].warps) continue;
+        if (launched[lead] || plans[lead].pool_stage || lanes[lead].warps || waves[lead].ng) continue;
         std::vector<uint32_t> members;
         for (uint32_t c = lead; c < nclass; ++c)
-            if (!launched[c] && !plans[c].pool_stage && !lanes[c].warps && plans[c].variant == plans[lead].variant &&
+            if (!launched[c] && !plans[c].pool_stage && !lanes[c].warps && !waves[c].ng && plans[c].variant == plans[lead].variant &&
                 plans[c].slots_smem == plans[lead].slots_smem)
                 members.push_back(c);
         if (members.size() < 2) continue;
@@ -562,6 +682,39 @@ int Ctx::run(const std::vector<Job>& jobs, uint64_t total, cudaStream_t st, uint
     for (uint32_t c = 0; c < nclass; ++c) {
         if (launched[c]) continue;
         const Plan& pl = plans[c];
+        if (waves[c].ng) {
+            const WavePlan& wp = waves[c];
+            const EngineArgs e = class_args(c);
+            WaveArgs a{};
+            a.jobs = e.jobs;
+            a.njobs = e.njobs;
+            a.total = e.total;
+            a.gidx_begin = e.gidx_begin;
+            a.ctrl = e.ctrl;
+            a.fail_bits = e.fail_bits;
+            a.job_failed = e.job_failed;
+            a.t0 = e.t0;
+            a.regions = d_slots + region[c];
+            a.region_bytes = wp.region_bytes;
+            a.map_off = wp.map_off;
+            a.wave = wp.wave;
+            a.min_wave = wp.min_wave;
+            a.stock = reinterpret_cast<uint32_t*>(a.regions + wp.regions_bytes);
+            a.gcache = wp.global_cache ? reinterpret_cast<uint16_t*>(a.regions + wp.regions_bytes + wp.stock_bytes)
+                                       : nullptr;
+            a.gcache_stride = wp.gcache_stride;
+            a.ng = wp.ng;
+            a.wg = wp.wg;
+            a.group_bytes = wp.group_bytes;
+            a.cache_off = wp.cache_off;
+            void* args[] = {&a};
+            if ((rc = cuda(cudaLaunchKernel(wave_kernel(wp.variant, wp.global_cache), dim3(wp.ctas),
+                                            dim3(wp.ng * wp.wg * 32), args, wp.smem_bytes, st),
+                           "wave engine launch")))
+                return rc;
+            ++kernels;
+            continue;
+        }
         if (lanes[c].warps) {
             const LanePlan& lp = lanes[c];
             const EngineArgs e = class_args(c);
@@ -676,6 +829,12 @@ const void* lane_kernel(int variant) {
                           : (const void*)cmc_lanes<false, true>;
 }
 
+const void* wave_kernel(int variant, bool global_cache) {
+    if (variant == 0)
+        return global_cache ? (const void*)cmc_waves<true, true> : (const void*)cmc_waves<true, false>;
+    return global_cache ? (const void*)cmc_waves<false, true> : (const void*)cmc_waves<false, false>;
+}
+
 // Every engine kernel may use up to the device's opt-in shared memory.  Set
 // once per device and never lowered, so launches of different plans -- and
 // graphs captured from them -- are valid whatever ran in between.
@@ -689,7 +848,8 @@ int engine_smem_cap(size_t optin) {
                          fused_engine_kernel(2, true), fused_engine_kernel(0, false),
                          fused_engine_kernel(1, false), fused_engine_kernel(2, false),
                          engine_kernel(0, true, true), engine_kernel(1, true, true),
-                         lane_kernel(0), lane_kernel(1), lane_kernel(2)};
+                         lane_kernel(0), lane_kernel(1), lane_kernel(2),
+                         wave_kernel(0, false), wave_kernel(0, true), wave_kernel(1, false), wave_kernel(1, true)};
     for (const void* fn : fns)
         if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(optin)) != cudaSuccess)
             return CMC_ECUDA;
@@ -861,7 +1021,7 @@ std::string Ctx::graph_key(const std::vector<Job>& jobs, const std::vector<uint3
     snprintf(b, sizeof b, "|%llu|%llu|%u/%u/%u/%u/%u/%d/%d/%d/%u/%u/%d|%p/%p/%p/%p/%p/%p/%p/%p",
              (unsigned long long)total, (unsigned long long)dev_cap, force_wg, force_ng,
              force_global_slots, force_walkers, max_slots_per_group, force_walker_ctas, force_isolate,
-             force_method, spin_limit, map_chains * 16 + fill_blocks, use_fused + 2 * force_lanes + 2 * 64 * force_pool, (void*)d_jobs, (void*)d_bits, (void*)d_out, (void*)d_slots,
+             force_method, spin_limit, map_chains * 16 + fill_blocks, use_fused + 2 * force_lanes + 128 * force_pool + 1024 * force_waves, (void*)d_jobs, (void*)d_bits, (void*)d_out, (void*)d_slots,
              (void*)d_ctrl, (void*)d_job_failed, (void*)h_failed, (void*)h_nf);
     return key + b;
 }
@@ -1228,6 +1388,8 @@ int cmc_set_option(cmc_ctx* ctx, const char* name, int64_t value) {
     else if (n == "global_slots" && (value == 0 || value == 1)) c->force_global_slots = uint32_t(value);
     else if (n == "method" && value >= -1 && value <= 2) c->force_method = int(value);
     else if (n == "lanes" && value >= -1 && value <= int64_t(cmc::kMaxLaneWarps)) c->force_lanes = int(value);
+    else if (n == "waves" && (value == -1 || value == 0 || value == 1 || value == 2 || value == 4 || value == 8))
+        c->force_waves = int(value);
     else if (n == "pool" && value >= -1 && value <= 1) c->force_pool = int(value);
     else if (n == "graph" && (value == 0 || value == 1)) c->use_graphs = int(value);
     else if (n == "fused" && (value == 0 || value == 1)) c->use_fused = int(value);
@@ -1296,7 +1458,12 @@ int cmc_plan_describe(const cmc_params* params, uint32_t count, uint32_t sms, ui
     int rc = c.make_job(*params, 0, count, 0, jobs[0]);
     cmc::Plan pl;
     if (!rc) rc = c.plan(jobs, pl);
-    if (!rc) c.plan_text += cmc::lanes_text(c.plan_lanes(jobs, pl));
+    if (!rc) {
+        cmc::LanePlan lanes;
+        cmc::WavePlan waves;
+        c.choose_engine(jobs, pl, lanes, waves);
+        c.plan_text += cmc::lanes_text(lanes) + cmc::waves_text(waves);
+    }
     snprintf(out, cap, "%s", (rc ? c.err : c.plan_text).c_str());
     if (rc) cmc::set_thread_error(c.err);
     return rc;

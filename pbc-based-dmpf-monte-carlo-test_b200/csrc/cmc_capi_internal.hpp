@@ -38,6 +38,20 @@ struct LanePlan {
     int variant = 0;            // as Plan::variant
     uint64_t region_bytes = 0;  // per lane
     uint64_t regions_bytes = 0, stock_bytes = 0;
+    double cycles = 0;          // estimated
+};
+
+// How a launch runs in the wave engine (cmc_waves.cu).
+struct WavePlan {
+    uint32_t ng = 0, wg = 0;    // groups per CTA (0: not used), warps per group
+    uint32_t wave = 0, min_wave = 1;  // trials per wave and group
+    uint32_t ctas = 0, smem_bytes = 0, group_bytes = 0, cache_off = 0, map_off = 0;
+    int variant = 0;            // as Plan::variant
+    bool global_cache = false;
+    uint32_t gcache_stride = 0;
+    uint64_t region_bytes = 0;  // per trial of a wave
+    uint64_t regions_bytes = 0, stock_bytes = 0, gcache_bytes = 0;
+    double cycles = 0;          // estimated
 };
 
 uint32_t choose_method(uint32_t h, uint64_t domain, double candidates, int force, bool may_allocate);
@@ -48,6 +62,7 @@ int engine_smem_cap(size_t optin);
 const void* engine_kernel(int variant, bool smem_slots, bool pooled = false);
 const void* fused_engine_kernel(int variant, bool smem_slots);
 const void* lane_kernel(int variant);
+const void* wave_kernel(int variant, bool global_cache);
 // Estimated cost of one trial in AES-block equivalents (seeds, map, 0.1 t for the walk).
 double job_cost(const Job& j);
 
@@ -112,6 +127,7 @@ struct Ctx {
     std::string graph_state;                 // "eager", "captured" or "replayed"
     int force_method = -1;  // -1 auto, 0 direct, 1 cache (shared if h <= 12, else global), 2 global cache
     int force_lanes = -1;   // lane engine: -1 auto, 0 off, N warps per CTA
+    int force_waves = -1;   // wave engine: -1 auto, 0 off, N groups per CTA
     int force_pool = -1;    // pooled direct passes: -1 auto, 0 off, 1 on where they apply
     bool plan_no_dfold = false;  // plan() re-run without room for direct passes' fold tables
     bool may_allocate = true;  // false: no global round cache, global slots only if unavoidable
@@ -128,6 +144,8 @@ struct Ctx {
     int make_job(const cmc_params& p, uint32_t first, uint32_t count, uint64_t base, Job& j);
     int plan(const std::vector<Job>& jobs, Plan& pl);
     LanePlan plan_lanes(const std::vector<Job>& jobs, const Plan& group) const;
+    WavePlan plan_waves(const std::vector<Job>& jobs, const Plan& group) const;
+    void choose_engine(const std::vector<Job>& jobs, const Plan& group, LanePlan& lanes, WavePlan& waves) const;
     int upload_jobs(const std::vector<Job>& jobs, cudaStream_t st);
     int run(const std::vector<Job>& jobs, uint64_t total, cudaStream_t st, uint32_t value_base,
             uint32_t* d_out, uint32_t* d_count, uint64_t out_cap, unsigned long long* job_failed,

@@ -12,10 +12,6 @@ constexpr uint32_t kMaxLaneWarps = 16;
 // Table reads per pass before a lane on known buckets sits one out: measured
 // at t = 64, 2^20 trials 20.5, 19.2, 19.0 and 19.1 ms with 1, 2, 4 and 8.
 constexpr uint32_t kLaneHops = 4;
-// Words of one trial's set-up record (LaneStock in cmc_lanes.cu), kept as
-// [word][32 records] per warp.
-constexpr uint32_t kLaneStockWords = 84;
-constexpr uint32_t kLaneStockBytes = kLaneStockWords * 32 * 4;
 
 struct LaneArgs {
     const Job* jobs;
@@ -29,7 +25,7 @@ struct LaneArgs {
     char* regions;                   // one table of B entries per lane that takes trials
     uint64_t region_bytes;
     uint32_t hops;                   // table reads per pass before a lane sits one out
-    uint32_t* stock;                 // kLaneStockBytes per warp
+    uint32_t* stock;                 // kRecordBlockBytes per warp
     uint32_t share;                  // lanes per warp that take trials (<= 32)
 };
 
