@@ -209,6 +209,56 @@ int Ctx::plan(const std::vector<Job>& jobs, Plan& pl) {
     // sub-partitions 0..2 (2 x 7, adding two beside the walker, is within 3%)
     if (pl.isolate && !force_wg) pl.wg = (any_cache || any_gcache) ? 6 : 4;
     if (pl.isolate && pl.nw > 4) pl.nw = 4;
+    const uint32_t budget = uint32_t(smem_optin) - kEngineTableBytes - kCtaSharedBytes;
+    uint32_t cap_ng = force_ng;
+    // Short launches (longer ones of these shapes run in the lane or wave engine)
+    // and callers that have this engine only: split all 15 warps beside the
+    // walker into as many groups as shared memory holds with enough walk slots
+    // -- 4 per group up to 28 -- and as there are trials for.  More, smaller
+    // groups overlap their serial set-ups and barriers.  Measured on B200
+    // against three 4-warp groups: t=30, N=2^8 0.121 against 0.211 ms (14 x 1),
+    // t=200, N=2^16 0.654 against 0.777 (7 x 2), t=600, N=2^24 1.46 against 1.75
+    // (5 x 3), t=1300 3.01 against 3.47 (3 x 5), t=300, k=4 (h=12) 1.68 against
+    // 1.92 (2 x 7).  Direct passes in pooled one-warp groups only where 13 or 14
+    // fit (t=280: 12 pooled groups 0.98 ms, 7 x 2 0.75).  Shared caches with long
+    // walks keep the walker isolated and take the split with most slots (t=700,
+    // N=2^16: 21 slots 1.22 ms, 16 slots 1.40).
+    const double per_sm = work / sms;
+    const bool short_launch = !may_allocate || group_only || per_sm <= 200;
+    if (short_launch && !force_wg && !force_ng && !force_walkers && force_isolate < 0 &&
+        !pl.walker_ctas && !any_gcache) {
+        const bool direct_pool = force_pool != 0 && !any_cache && !wide_domain;
+        auto slots_at = [&](uint32_t ng, uint32_t bytes) {
+            return ng * bytes > budget
+                       ? 0u
+                       : ng * std::min<uint32_t>({(budget - ng * bytes) / pl.slot_stride / ng, 32 / ng,
+                                                  max_slots_per_group});
+        };
+        if (any_cache ? avg_probe_work >= 512 : avg_probe_work >= 1500) {
+            uint32_t most = 0;
+            for (uint32_t ng : {2u, 3u, 4u, 6u}) {
+                const uint32_t s = slots_at(ng, pl.group_bytes);
+                if (any_cache && s > most) {
+                    most = s;
+                    cap_ng = ng;
+                    pl.wg = 12 / ng;
+                }
+            }
+        } else {
+            for (uint32_t wg : {1u, 2u, 3u, 5u, 7u, 15u}) {
+                const uint32_t ng = std::min<uint32_t>(kMaxGroups, 15 / wg);
+                const uint32_t pool = pool_group_bytes(round_up(max_cand * entry, 16),
+                                                       max_h <= 10 ? fold_table_bytes(max_h) : 0);
+                if (ng > 1 && ng > 2 * per_sm + 1) continue;
+                if (wg == 1 && direct_pool && slots_at(ng, pool) < 28 && slots_at(13, pool) < 26) continue;
+                if (!(wg == 1 && direct_pool) && slots_at(ng, pl.group_bytes) < std::min(4 * ng, 28u)) continue;
+                pl.wg = wg;
+                pl.isolate = 0;
+                cap_ng = ng;
+                break;
+            }
+        }
+    }
     // Pooled direct passes (producer_pooled): one-warp groups whose jobs all
     // use direct passes with 16-bit halves; each group then holds three trials'
     // headers and staged maps.  Dropped below if the walk slots go global.
@@ -223,10 +273,9 @@ int Ctx::plan(const std::vector<Job>& jobs, Plan& pl) {
         pl.pool_fold = max_h <= 10 ? fold_table_bytes(max_h) : 0;
         pl.group_bytes = pool_group_bytes(pl.pool_stage, pl.pool_fold);  // its own fold, if any
     }
-    const uint32_t budget = uint32_t(smem_optin) - kEngineTableBytes - kCtaSharedBytes;
     auto groups_for = [&](uint32_t nw) {
         uint32_t ng = std::min<uint32_t>(kMaxGroups, (16 - nw) / pl.wg);
-        if (force_ng) ng = std::min(ng, force_ng);
+        if (cap_ng) ng = std::min(ng, cap_ng);
         while (ng > 1 && ng * pl.group_bytes > budget) --ng;
         return ng;
     };
@@ -274,7 +323,9 @@ int Ctx::plan(const std::vector<Job>& jobs, Plan& pl) {
         // a walker beside ALU-bound producers issues slower: ~800 cycles per
         // shared probe (measured at t=500, k=4), ~300 when isolated
         const double walk_smem = pl.slots_smem ? pl.ns / (probes * (pl.isolate ? 300.0 : 800.0)) : 0.0;
-        const double walk_global = ns_g / (probes * 3000.0);
+        // (short launches: ~4500, measured at t=1500, N=2^16, where 10 shared
+        // slots give 3.74 ms and 128 global ones 5.17)
+        const double walk_global = ns_g / (probes * (short_launch ? 4500.0 : 3000.0));
         const bool keep_smem = pl.slots_smem && (!may_allocate || walk_smem >= 1.4 * produce ||
                                                  walk_smem >= walk_global);
         if (!keep_smem) {
@@ -513,10 +564,13 @@ void Ctx::choose_engine(const std::vector<Job>& jobs, const Plan& group, LanePla
         lanes = plan_lanes(jobs, group);
         return;
     }
-    uint64_t count = 0;
-    for (const Job& j : jobs) count += j.count;
-    // a CTA without a full wave of its groups' threads gains nothing
-    if (group_options || force_waves > 0 || count < 2ull * sms) return;
+    uint64_t count = 0, items = 0;
+    for (const Job& j : jobs) {
+        count += j.count;
+        items = std::max<uint64_t>(items, j.pnum);
+    }
+    // the smallest launches gain nothing: not worth the estimates
+    if (group_options || force_waves > 0 || (count < 4ull * sms && items < 128)) return;
     const double limit = group_cycles(jobs, group, sms);
     if (force_waves < 0) waves = plan_waves(jobs, group);
     if (force_lanes < 0 && count >= 16ull * sms) lanes = plan_lanes(jobs, group);

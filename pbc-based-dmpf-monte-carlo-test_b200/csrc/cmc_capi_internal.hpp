@@ -130,6 +130,7 @@ struct Ctx {
     int force_waves = -1;   // wave engine: -1 auto, 0 off, N groups per CTA
     int force_pool = -1;    // pooled direct passes: -1 auto, 0 off, 1 on where they apply
     bool plan_no_dfold = false;  // plan() re-run without room for direct passes' fold tables
+    bool group_only = false;   // the caller has no lane or wave engine (a server's launches)
     bool may_allocate = true;  // false: no global round cache, global slots only if unavoidable
     uint32_t spin_limit = 1u << 26;
     uint32_t map_chains = 0;  // lookup chains per lane from a round cache (0: automatic)
