@@ -127,13 +127,48 @@ __device__ __forceinline__ uint32_t next_digit(uint64_t& walk, uint64_t& rnd, ui
     return d;
 }
 
-// The next 32 digits, two bits each, lowest first.
-__device__ __forceinline__ uint64_t next_digits(uint64_t& walk, uint64_t& rnd, uint32_t k) {
-    uint64_t d = 0;
-#pragma unroll 4
-    for (uint32_t i = 0; i < 32; ++i) d |= (uint64_t)next_digit(walk, rnd, k) << (2 * i);
-    return d;
-}
+// The digits of a walk decoded ahead, eight at a time: one 64-bit division by
+// k^8 and eight 16-bit ones instead of eight 64-bit ones.  A randomness below
+// k^8 gives its last digits (as long as it is k or more) and is replaced.
+struct Digits {
+    uint64_t walk = 0, rnd = 0;
+    uint64_t buf = 0;  // n digits of two bits, the next one lowest
+    uint32_t n = 0;
+
+    // Appends up to eight digits (n <= 24 before).
+    __device__ __forceinline__ void block(uint32_t k) {
+        const uint32_t all = k == 3 ? 6561u : k == 2 ? 256u : 65536u;
+        // floor(rnd / 3^8) for every 64-bit rnd: 0x9fd1... = ceil(2^76 / 3^8), within 2^12 / 3^8 of it
+        const uint64_t q8 = k == 3 ? __umul64hi(rnd, 0x9fd1cd5aa3cca6d8ULL) >> 12 : rnd >> (k == 2 ? 8 : 16);
+        const bool full = rnd >= all;
+        uint32_t r = full ? (uint32_t)rnd - (uint32_t)q8 * all : (uint32_t)rnd;
+        uint32_t word = 0, m = 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            m += r >= k;
+            // 21846 = ceil(2^16 / 3) divides r < 2^15 by 3
+            const uint32_t q = k == 3 ? (r * 21846u) >> 16 : r >> (k >> 1);
+            word |= (r - q * k) << (2 * i);
+            r = q;
+        }
+        m = full ? 8u : m;
+        buf |= (uint64_t)(word & ((1u << (2 * m)) - 1u)) << (2 * n);
+        n += m;
+        rnd = q8;
+        if (!full) rnd = splitmix(walk);
+    }
+    // At least 17 digits.
+    __device__ __forceinline__ void top_up(uint32_t k) {
+        while (n <= 16) block(k);
+    }
+    __device__ __forceinline__ uint32_t next(uint32_t k) {
+        while (n == 0) block(k);
+        const uint32_t d = (uint32_t)buf & 3u;
+        buf >>= 2;
+        --n;
+        return d;
+    }
+};
 
 // The buckets of an item that its trial has evaluated so far (kUnknown for the
 // others) and, packed with its ordinal, the table entry that holds it.  The

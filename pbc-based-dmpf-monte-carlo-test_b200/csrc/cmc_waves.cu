@@ -166,11 +166,14 @@ __device__ __forceinline__ bool wave_map(const Job& J, const uint32_t* rec, cons
 
 // The walks of a warp's trials, one per lane (`active`); returns whether this
 // lane's failed.  A step reads one bin per lane, all at the same place of the
-// loop.  What bounds it is latency: the table read and the chain of
-// instructions behind it, so the walk's digits are decoded ahead, 32 at a time
-// and for all lanes together (their 64-bit divisions took most of a step when
-// each lane decoded its next one: 3,500 cycles a step with 32 lanes), and an
-// item's entry is its buckets with one field replaced.
+// loop, and its two outcomes (item placed, item evicted) are selects, not
+// branches.  A walk alone is bound by latency, the table read and the chain of
+// instructions behind it; beside other groups' fills by the ALU pipe, which
+// the fills use to 85 %.  The walk's digits are therefore decoded ahead, for
+// all lanes together, and an item that returns to the bin it left costs no
+// read (t = 1024, N = 2^20: 250 ALU instructions per step with 64-bit digit
+// divisions and a loop over returning items, 3,500 cycles a step with 32 lanes
+// and branches).
 template <bool NARROW>
 __device__ __forceinline__ bool walk_bgh(const Job& J, bool active, uint64_t walk, uint64_t rnd, char* region,
                                          uint32_t map_off, uint32_t& steps) {
@@ -181,40 +184,27 @@ __device__ __forceinline__ bool walk_bgh(const Job& J, bool active, uint64_t wal
     const Entry* map = reinterpret_cast<const Entry*>(region + map_off);
     const uint32_t k = J.k, last = J.pnum - 1, kick = J.kick;
     const bool four = k == 4;
-    uint32_t item = 0, cur = 0, count = 0, left = 0, left2 = 0;
-    uint64_t digits = 0, digits2 = 0;
-    bool failed = false;
-    auto digit = [&]() {
-        if (left == 0) {
-            if (left2 == 0) digits2 = next_digits(walk, rnd, k);
-            digits = digits2;
-            left = 32;
-            left2 = 0;
-        }
-        const uint32_t d = (uint32_t)digits & 3u;
-        digits >>= 2;
-        --left;
-        return d;
-    };
+    uint32_t item = 0, cur = 0, count = 0, which = 0, bin = 0;
+    bool failed = false, again = false;
+    Digits digits;
+    digits.walk = walk;
+    digits.rnd = rnd;
     ItemT it{};
-    Entry ahead{};  // the next item's buckets
-    uint32_t which = 0, bin = 0;
+    Entry ahead{}, mine{};  // the next item's buckets; what this lane wrote last
     if (active) {
         it = ItemT::from(ItemT::load(map));
         ahead = ItemT::load(map + 1);  // t >= 3
-        which = digit();
+        which = digits.next(k);
         bin = it.get(which);
     }
     for (uint32_t s = 0; __any_sync(kFull, active); ++s) {
-        if ((s & 15u) == 0 && active && left2 == 0) {
-            digits2 = next_digits(walk, rnd, k);
-            left2 = 32;
-        }
+        if ((s & 7u) == 0 && active) digits.top_up(k);
         if (!active) continue;
-        const Entry old = ItemT::load(bins + bin);
-        Entry mine = it.pack(cur, which, four);
+        Entry old = mine;  // an item that returns to the bin it left finds the item that evicted it
+        if (!again) old = ItemT::load(bins + bin);
+        mine = it.pack(cur, which, four);
         ++steps;
-        which = digit();
+        which = digits.next(k);
         const bool placed = ItemT::empty(old);
         uint32_t copy;
         it.unpack(old, bin, four, cur, copy);
@@ -226,17 +216,17 @@ __device__ __forceinline__ bool walk_bgh(const Job& J, bool active, uint64_t wal
         count = placed ? 0u : count + 1;
         if (placed) ahead = ItemT::load(map + min(item + 1, last));
         failed = count > kick;
-        while (which == copy && !failed) {
-            // the copy it was evicted from: it takes this bin back
+        if (which == copy && !failed) {
             ++steps;
             const Entry back = it.pack(cur, which, four);
             it.unpack(mine, bin, four, cur, copy);
             mine = back;
-            which = digit();
+            which = digits.next(k);
             failed = ++count > kick;
         }
         ItemT::store(bins + bin, mine);
         active = active && !failed;
+        again = which == copy;
         bin = it.get(which);
     }
     return failed;
