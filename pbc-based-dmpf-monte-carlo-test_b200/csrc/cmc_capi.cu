@@ -34,7 +34,8 @@ template <bool NARROW, bool GC>
 __global__ void cmc_waves(const WaveArgs a);
 __global__ void cmc_compact_failures(const uint32_t* bits, uint64_t nbits, uint32_t value_base,
                                      uint32_t* out, uint32_t* count, uint64_t cap,
-                                     const unsigned long long* nbits_dev);
+                                     const unsigned long long* nbits_dev,
+                                     CallResult* result, const Ctrl* ctrl, uint32_t nctrl);
 __global__ void cmc_selftest(const uint32_t* t0, const uint32_t* fips_rk, uint32_t* out,
                              uint32_t r256);
 
@@ -586,7 +587,7 @@ void Ctx::choose_engine(const std::vector<Job>& jobs, const Plan& group, LanePla
 int Ctx::run(const std::vector<Job>& jobs, uint64_t total, cudaStream_t st, uint32_t value_base,
              uint32_t* d_out, uint32_t* d_count, uint64_t out_cap_now,
              unsigned long long* job_failed, unsigned long long* job_done,
-             const std::vector<uint32_t>* bounds_in) {
+             const std::vector<uint32_t>* bounds_in, bool read_back) {
     // launch checks below read cudaGetLastError: start from a clean slate (an
     // earlier non-fatal error, e.g. of a timing query, is not this launch's)
     cudaGetLastError();
@@ -640,21 +641,22 @@ int Ctx::run(const std::vector<Job>& jobs, uint64_t total, cudaStream_t st, uint
     }
     plan_text = fuse ? "fused(" + std::to_string(nclass) + ") " + text : text;
     const size_t words = (total + 31) / 32;
-    int rc = grow(d_bits, bits_cap, words, "failure bitmap");
+    int rc = bitmap(words);
     if (rc) return rc;
+    uint32_t* const bits = d_bits + kCtrlWords;
     // walk slots, then the groups' round caches, per pool region
     if (pool && (rc = grow(d_slots, slots_cap, size_t(pool), "slot and cache pool"))) {
         if (rc != CMC_ENOMEM || (force_lanes == 0 && force_waves == 0)) return rc;
         // no room for the tables of the lane or wave engine: the group engine needs less
         const int kept[2] = {force_lanes, force_waves};
         force_lanes = force_waves = 0;
-        rc = run(jobs, total, st, value_base, d_out, d_count, out_cap_now, job_failed, job_done, bounds_in);
+        rc = run(jobs, total, st, value_base, d_out, d_count, out_cap_now, job_failed, job_done, bounds_in,
+                 read_back);
         force_lanes = kept[0];
         force_waves = kept[1];
         return rc;
     }
-    if ((rc = cuda(cudaMemsetAsync(d_ctrl, 0, nclass * sizeof(Ctrl), st), "memset ctrl"))) return rc;
-    if ((rc = cuda(cudaMemsetAsync(d_bits, 0, words * 4, st), "memset bitmap"))) return rc;
+    if ((rc = cuda(cudaMemsetAsync(d_bits, 0, (kCtrlWords + words) * 4, st), "memset ctrl and bitmap"))) return rc;
     // timing events stay out of captured graphs: a replay records them
     // around the graph launch instead
     if (!capturing && (rc = cuda(cudaEventRecord(ev_start, st), "event"))) return rc;
@@ -669,7 +671,7 @@ int Ctx::run(const std::vector<Job>& jobs, uint64_t total, cudaStream_t st, uint
         a.gidx_begin = jobs[bounds[c]].trial_base;
         a.total = bounds[c + 1] < jobs.size() ? jobs[bounds[c + 1]].trial_base : total;
         a.ctrl = d_ctrl + c;
-        a.fail_bits = d_bits;
+        a.fail_bits = bits;
         a.job_failed = job_failed;
         a.job_done = job_done;
         a.gslots = pl.slots_smem ? nullptr : base;
@@ -819,8 +821,8 @@ int Ctx::run(const std::vector<Job>& jobs, uint64_t total, cudaStream_t st, uint
     }
     if (!capturing && (rc = cuda(cudaEventRecord(ev_stop, st), "event"))) return rc;
     if (d_out) {
-        cmc_compact_failures<<<1, 1024, 0, st>>>(d_bits, total, value_base, d_out, d_count, out_cap_now,
-                                                 nullptr);
+        cmc_compact_failures<<<1, 1024, 0, st>>>(bits, total, value_base, d_out, d_count, out_cap_now,
+                                                 nullptr, read_back ? d_result : nullptr, d_ctrl, nclass);
         if ((rc = cuda(cudaGetLastError(), "compaction launch"))) return rc;
         ++kernels;
     }
@@ -829,11 +831,23 @@ int Ctx::run(const std::vector<Job>& jobs, uint64_t total, cudaStream_t st, uint
     return CMC_OK;
 }
 
+// Room for the control blocks and a failure bitmap of `words` words.
+int Ctx::bitmap(size_t words) {
+    const int rc = grow(d_bits, bits_cap, kCtrlWords + words, "failure bitmap");
+    d_ctrl = reinterpret_cast<Ctrl*>(d_bits);
+    return rc;
+}
+
 int Ctx::check_ctrl() {
+    if (!d_ctrl) return CMC_OK;  // no launch since an allocation failed
     Ctrl c[kMaxClasses]{};
     const uint32_t n = std::max<uint32_t>(1, ctrl_count);
     int rc = cuda(cudaMemcpy(c, d_ctrl, n * sizeof(Ctrl), cudaMemcpyDeviceToHost), "read ctrl");
-    if (rc) return rc;
+    return rc ? rc : check_ctrl(c);
+}
+
+int Ctx::check_ctrl(const Ctrl* c) {
+    const uint32_t n = std::max<uint32_t>(1, ctrl_count);
     Ctrl sum{};
     for (uint32_t i = 0; i < n; ++i) {
         if (c[i].error && !sum.error) {
@@ -938,8 +952,13 @@ int Ctx::init(int dev) {
     if ((rc = cuda(cudaMemcpy(d_t0, t0, sizeof t0, cudaMemcpyHostToDevice), "upload T0"))) return rc;
     if ((rc = cuda(cudaMemcpy(d_t0 + 256, fips, sizeof fips, cudaMemcpyHostToDevice), "upload KAT key")))
         return rc;
-    size_t c1 = 0;
-    if ((rc = grow(d_ctrl, c1, kMaxClasses, "ctrl"))) return rc;
+    if ((rc = bitmap(0))) return rc;
+    if (cudaHostAlloc((void**)&h_result, sizeof(CallResult), cudaHostAllocMapped) != cudaSuccess ||
+        cudaHostGetDevicePointer((void**)&d_result, h_result, 0) != cudaSuccess ||
+        cudaHostAlloc((void**)&h_job, sizeof(Job), cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();
+        return fail(CMC_ENOMEM, "pinned call buffers");
+    }
     const uint32_t kat_smem = kEngineTableBytes;
     if ((rc = cuda(cudaFuncSetAttribute((const void*)cmc_selftest,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, kat_smem),
@@ -961,7 +980,6 @@ Ctx::~Ctx() {
     if (device < 0) return;  // a planner that never touched a device holds nothing to free
     cudaSetDevice(device);
     cudaFree(d_t0);
-    cudaFree(d_ctrl);
     cudaFree(d_jobs);
     cudaFree(d_bits);
     cudaFree(d_out);
@@ -971,7 +989,8 @@ Ctx::~Ctx() {
     cudaFree(d_key);
     for (GraphEntry& g : graphs) cudaGraphExecDestroy(g.exec);
     cudaFreeHost(h_failed);
-    cudaFreeHost(h_nf);
+    cudaFreeHost(h_result);
+    cudaFreeHost(h_job);
     if (ev_start) cudaEventDestroy(ev_start);
     if (ev_stop) cudaEventDestroy(ev_stop);
     if (stream) cudaStreamDestroy(stream);
@@ -998,19 +1017,24 @@ int Ctx::launch_host(const cmc_params& p, const uint32_t key[44], uint32_t first
     std::vector<Job> jobs(1);
     if ((rc = make_job(p, first, count, 0, jobs[0]))) return rc;
     std::memcpy(jobs[0].batch_rk, key, 44 * 4);
-    if ((rc = upload_jobs(jobs, st))) return rc;
+    if ((rc = grow(d_jobs, jobs_cap, 1, "job table"))) return rc;
+    *h_job = jobs[0];
+    if ((rc = cuda(cudaMemcpyAsync(d_jobs, h_job, sizeof(Job), cudaMemcpyHostToDevice, st), "upload job"))) return rc;
     if ((rc = grow(d_out, out_cap, size_t(count) + 1, "failure list"))) return rc;
-    if ((rc = run(jobs, count, st, first, d_out, d_out + count, count, nullptr, nullptr))) return rc;
-    uint32_t nf = 0;
-    if ((rc = cuda(cudaMemcpyAsync(&nf, d_out + count, 4, cudaMemcpyDeviceToHost, st), "read count")))
-        return rc;
+    // one synchronisation: the compaction writes count, control block and the
+    // first offsets to host memory (t = 16, 256 trials: three copies and their
+    // synchronisations took 20 of a call's 77 us)
+    if ((rc = run(jobs, count, st, first, d_out, d_out + count, count, nullptr, nullptr, nullptr, true))) return rc;
     if ((rc = cuda(cudaStreamSynchronize(st), "launch sync"))) return rc;
-    if ((rc = check_ctrl())) return rc;
+    if ((rc = check_ctrl(h_result->ctrl))) return rc;
+    const uint32_t nf = h_result->count;
     if (nf > count) return fail(CMC_ERANGE, "GPU failure count out of range");
-    if (nf && (rc = cuda(cudaMemcpyAsync(out, d_out, size_t(nf) * 4, cudaMemcpyDeviceToHost, st),
-                         "read offsets")))
+    std::memcpy(out, h_result->offsets, size_t(std::min(nf, kInlineOffsets)) * 4);
+    if (nf > kInlineOffsets &&
+        (rc = cuda(cudaMemcpy(out + kInlineOffsets, d_out + kInlineOffsets, size_t(nf - kInlineOffsets) * 4,
+                              cudaMemcpyDeviceToHost),
+                   "read offsets")))
         return rc;
-    if (nf && (rc = cuda(cudaStreamSynchronize(st), "offsets sync"))) return rc;
     *nfailed = nf;
     return CMC_OK;
 }
@@ -1072,11 +1096,11 @@ std::string Ctx::graph_key(const std::vector<Job>& jobs, const std::vector<uint3
         key += b;
     }
     for (uint32_t x : bounds) key += std::to_string(x) + ",";
-    snprintf(b, sizeof b, "|%llu|%llu|%u/%u/%u/%u/%u/%d/%d/%d/%u/%u/%d|%p/%p/%p/%p/%p/%p/%p/%p",
+    snprintf(b, sizeof b, "|%llu|%llu|%u/%u/%u/%u/%u/%d/%d/%d/%u/%u/%d|%p/%p/%p/%p/%p/%p/%p",
              (unsigned long long)total, (unsigned long long)dev_cap, force_wg, force_ng,
              force_global_slots, force_walkers, max_slots_per_group, force_walker_ctas, force_isolate,
              force_method, spin_limit, map_chains * 16 + fill_blocks, use_fused + 2 * force_lanes + 128 * force_pool + 1024 * force_waves, (void*)d_jobs, (void*)d_bits, (void*)d_out, (void*)d_slots,
-             (void*)d_ctrl, (void*)d_job_failed, (void*)h_failed, (void*)h_nf);
+             (void*)d_ctrl, (void*)d_job_failed, (void*)h_failed);
     return key + b;
 }
 
@@ -1201,21 +1225,15 @@ int Ctx::run_jobs(const cmc_job* in, uint32_t n, uint64_t* out_failed, uint32_t*
         }
         h_failed_cap = n;
     }
-    if (!h_nf && cudaHostAlloc((void**)&h_nf, 4, cudaHostAllocDefault) != cudaSuccess) {
-        cudaGetLastError();
-        return fail(CMC_ENOMEM, "pinned count");
-    }
     // The device side of the call: counters, the engine launches, the
     // compaction and the read-back into pinned memory.
     auto enqueue = [&]() -> int {
         int r = cuda(cudaMemsetAsync(d_job_failed, 0, n * sizeof(unsigned long long), st), "memset counters");
         if (r) return r;
-        if ((r = run(jobs, total, st, 0, d_out, d_out + dev_cap, dev_cap, d_job_failed, nullptr, &bounds)))
+        if ((r = run(jobs, total, st, 0, d_out, d_out + dev_cap, dev_cap, d_job_failed, nullptr, &bounds, true)))
             return r;
-        if ((r = cuda(cudaMemcpyAsync(h_failed, d_job_failed, n * sizeof(unsigned long long),
-                                      cudaMemcpyDeviceToHost, st), "read counters")))
-            return r;
-        return cuda(cudaMemcpyAsync(h_nf, d_out + dev_cap, 4, cudaMemcpyDeviceToHost, st), "read count");
+        return cuda(cudaMemcpyAsync(h_failed, d_job_failed, n * sizeof(unsigned long long),
+                                    cudaMemcpyDeviceToHost, st), "read counters");
     };
     // A call shape seen before is captured into a CUDA graph on its second
     // call and replayed from the third: the job table is uploaded by copy
@@ -1275,9 +1293,9 @@ int Ctx::run_jobs(const cmc_job* in, uint32_t n, uint64_t* out_failed, uint32_t*
     }
     if (use_graphs) plan_text += " graph=" + graph_state;
     if ((rc = cuda(cudaStreamSynchronize(st), "batched sync"))) return rc;
-    if ((rc = check_ctrl())) return rc;
+    if ((rc = check_ctrl(h_result->ctrl))) return rc;
     std::vector<unsigned long long> failed(h_failed, h_failed + n);
-    const uint32_t nf = *h_nf;
+    const uint32_t nf = h_result->count;
     uint64_t sum = 0;
     for (uint32_t i = 0; i < n; ++i) {
         out_failed[order[i]] = failed[i];
@@ -1287,8 +1305,11 @@ int Ctx::run_jobs(const cmc_job* in, uint32_t n, uint64_t* out_failed, uint32_t*
     if (out_total) *out_total = nf;
     if (out_offsets && nf) {
         const uint64_t m = std::min<uint64_t>(nf, dev_cap);
-        std::vector<uint32_t> g(m);
-        if ((rc = cuda(cudaMemcpy(g.data(), d_out, m * 4, cudaMemcpyDeviceToHost), "read failures"))) return rc;
+        std::vector<uint32_t> g(h_result->offsets, h_result->offsets + std::min<uint64_t>(m, kInlineOffsets));
+        if (m > kInlineOffsets) {
+            g.resize(m);
+            if ((rc = cuda(cudaMemcpy(g.data(), d_out, m * 4, cudaMemcpyDeviceToHost), "read failures"))) return rc;
+        }
         // global index -> (original job, offset); global order is job-major in
         // the heavy-first order, so regroup by the caller's job order
         std::vector<std::pair<uint32_t, uint32_t>> pairs(m);

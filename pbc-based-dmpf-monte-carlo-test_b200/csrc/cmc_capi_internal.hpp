@@ -15,6 +15,10 @@ namespace cmc {
 constexpr uint32_t kMaxClasses = 16;  // plan classes per batched call
 static_assert(kMaxClasses <= kMaxFusedClasses, "every class fits a fused launch");
 
+constexpr uint32_t kCtrlWords = 320;  // room for kMaxClasses control blocks
+static_assert(kMaxClasses * sizeof(Ctrl) <= kCtrlWords * 4, "control blocks fit their room");
+static_assert(kMaxClasses <= kResultCtrls, "a result holds every class's control block");
+
 struct Plan {
     uint32_t ng = 0, wg = 0, ns = 0, nw = 1;
     uint32_t walker_ctas = 0;  // > 0: split engine with this many walker CTAs
@@ -82,12 +86,15 @@ struct Ctx {
     cudaStream_t user_stream = nullptr;  // cmc_set_stream override
     cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
     uint32_t* d_t0 = nullptr;  // T0 table, FIPS KAT schedule, self-test output
-    Ctrl* d_ctrl = nullptr;      // one control block per plan class of a launch
+    Ctrl* d_ctrl = nullptr;      // one control block per plan class of a launch, at the head of d_bits
     uint32_t ctrl_count = 1;     // control blocks the last run used
     Job* d_jobs = nullptr;
     size_t jobs_cap = 0;
-    uint32_t* d_bits = nullptr;
+    uint32_t* d_bits = nullptr;  // kCtrlWords of control blocks, then the failure bitmap
     size_t bits_cap = 0;
+    CallResult* h_result = nullptr;  // mapped host memory: what a synchronous call reads back
+    CallResult* d_result = nullptr;  // its device address
+    Job* h_job = nullptr;            // pinned staging of cmc_launch's one job
     uint32_t* d_out = nullptr;
     size_t out_cap = 0;
     char* d_slots = nullptr;
@@ -123,7 +130,6 @@ struct Ctx {
     std::vector<std::string> graph_seen;
     unsigned long long* h_failed = nullptr;  // pinned per-job counts of the last batched call
     size_t h_failed_cap = 0;
-    uint32_t* h_nf = nullptr;                // pinned failure count of the last batched call
     std::string graph_state;                 // "eager", "captured" or "replayed"
     int force_method = -1;  // -1 auto, 0 direct, 1 cache (shared if h <= 12, else global), 2 global cache
     int force_lanes = -1;   // lane engine: -1 auto, 0 off, N warps per CTA
@@ -150,8 +156,11 @@ struct Ctx {
     int upload_jobs(const std::vector<Job>& jobs, cudaStream_t st);
     int run(const std::vector<Job>& jobs, uint64_t total, cudaStream_t st, uint32_t value_base,
             uint32_t* d_out, uint32_t* d_count, uint64_t out_cap, unsigned long long* job_failed,
-            unsigned long long* job_done, const std::vector<uint32_t>* class_bounds = nullptr);
+            unsigned long long* job_done, const std::vector<uint32_t>* class_bounds = nullptr,
+            bool read_back = false);
     int check_ctrl();
+    int check_ctrl(const Ctrl* blocks);
+    int bitmap(size_t words);
     int launch_host(const cmc_params& p, const uint32_t key[44], uint32_t first, uint32_t count,
                     uint32_t* out, uint32_t* nfailed);
     int launch_device(const cmc_params& p, const uint32_t* d_key, uint32_t first, uint32_t count,

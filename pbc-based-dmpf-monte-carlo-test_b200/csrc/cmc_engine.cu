@@ -1506,14 +1506,22 @@ __global__ void __launch_bounds__(512, 1) cmc_engine_fused(const __grid_constant
 
 // Ordered failure list from the bitmap: one CTA, block-wide exclusive scan.
 // out[i] = value_base + (index of the i-th set bit) for i < cap; *count = the
-// number of set bits.
+// number of set bits.  With `result` (host memory), the same there, and the
+// launch's nctrl control blocks.
 __global__ void __launch_bounds__(1024) cmc_compact_failures(const uint32_t* __restrict__ bits,
                                                              uint64_t nbits, uint32_t value_base,
                                                              uint32_t* __restrict__ out,
                                                              uint32_t* __restrict__ count,
                                                              uint64_t cap,
-                                                             const unsigned long long* nbits_dev) {
+                                                             const unsigned long long* nbits_dev,
+                                                             CallResult* result, const Ctrl* ctrl,
+                                                             uint32_t nctrl) {
     __shared__ uint32_t warp_sums[32];
+    if (result) {
+        const uint32_t* src = reinterpret_cast<const uint32_t*>(ctrl);
+        uint32_t* dst = reinterpret_cast<uint32_t*>(result->ctrl);
+        for (uint32_t i = threadIdx.x; i < nctrl * sizeof(Ctrl) / 4; i += blockDim.x) dst[i] = src[i];
+    }
     if (nbits_dev) nbits = *nbits_dev;
     const uint64_t words = (nbits + 31) / 32;
     const uint64_t per = (words + blockDim.x - 1) / blockDim.x;
@@ -1536,7 +1544,10 @@ __global__ void __launch_bounds__(1024) cmc_compact_failures(const uint32_t* __r
             if (lane >= (uint32_t)o) s += u;
         }
         if (lane < nw) warp_sums[lane] = s - v;  // exclusive
-        if (lane == nw - 1) *count = s;
+        if (lane == nw - 1) {
+            *count = s;
+            if (result) result->count = s;
+        }
     }
     __syncthreads();
     uint32_t at = warp_sums[warp] + incl - mine;
@@ -1545,7 +1556,9 @@ __global__ void __launch_bounds__(1024) cmc_compact_failures(const uint32_t* __r
         while (b) {
             const int i = __ffs(b) - 1;
             b &= b - 1;
-            if (at < cap) out[at] = value_base + (uint32_t)(w * 32 + i);
+            const uint32_t v = value_base + (uint32_t)(w * 32 + i);
+            if (at < cap) out[at] = v;
+            if (result && at < kInlineOffsets) result->offsets[at] = v;
             ++at;
         }
     }

@@ -65,6 +65,17 @@ struct Ctrl {
     unsigned int groups_done;              // split engine: producer groups finished
 };
 
+// What the host reads back from a call: written by cmc_compact_failures into
+// mapped host memory, so that a call ends with one stream synchronisation and
+// no copy unless more than kInlineOffsets trials failed.
+constexpr uint32_t kResultCtrls = 16;
+constexpr uint32_t kInlineOffsets = 2048;
+struct CallResult {
+    Ctrl ctrl[kResultCtrls];
+    uint32_t count, pad;
+    uint32_t offsets[kInlineOffsets];
+};
+
 // What a nonzero Ctrl::error means, for the host's error message.
 inline const char* ctrl_error_text(unsigned int error) {
     switch (error) {

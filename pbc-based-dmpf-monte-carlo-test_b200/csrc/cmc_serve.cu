@@ -48,7 +48,8 @@ namespace cmc {
 
 __global__ void cmc_compact_failures(const uint32_t* bits, uint64_t nbits, uint32_t value_base,
                                      uint32_t* out, uint32_t* count, uint64_t cap,
-                                     const unsigned long long* nbits_dev);
+                                     const unsigned long long* nbits_dev,
+                                     CallResult* result, const Ctrl* ctrl, uint32_t nctrl);
 
 namespace {
 
@@ -668,7 +669,7 @@ struct Server {
             return rc;
         if ((rc = cuda(cudaEventRecord(b.e1, st), "event"))) return rc;
         cmc_compact_failures<<<1, 1024, 0, st>>>(b.d_bits, 0, 0, b.d_list, b.d_list + max_iter_trials,
-                                                 max_iter_trials, b.d_total);
+                                                 max_iter_trials, b.d_total, nullptr, nullptr, 0);
         if ((rc = cuda(cudaGetLastError(), "compaction launch"))) return rc;
         if ((rc = cuda(cudaMemcpyAsync(b.h_info, b.d_info, grants.size() * sizeof(GrantInfo),
                                        cudaMemcpyDeviceToHost, st), "read grant info")))
