@@ -125,20 +125,23 @@ __device__ __forceinline__ uint32_t sub_word(const Lanes& L, uint32_t v) {
            (sbox_byte(L, v >> 8) << 8) | sbox_byte(L, v);
 }
 
-// FIPS-197 key schedule from four big-endian key words (cuckoo_bench.cu:136-149).
+// FIPS-197 key schedule from four big-endian key words (cuckoo_bench.cu:136-149);
+// the running words stay in registers, rk is only written.
 __device__ __forceinline__ void expand_key(const Lanes& L, uint32_t a, uint32_t b, uint32_t c,
                                            uint32_t d, uint32_t* rk) {
     rk[0] = a; rk[1] = b; rk[2] = c; rk[3] = d;
     uint32_t rcon = 1;
 #pragma unroll 1
     for (int i = 4; i < 44; i += 4) {
-        const uint32_t v = rk[i - 1];
-        const uint32_t t = sub_word(L, (v << 8) | (v >> 24)) ^ (rcon << 24);
+        a ^= sub_word(L, (d << 8) | (d >> 24)) ^ (rcon << 24);
         rcon = (rcon << 1) ^ ((rcon & 0x80u) ? 0x1bu : 0u);
-        rk[i] = rk[i - 4] ^ t;
-        rk[i + 1] = rk[i - 3] ^ rk[i];
-        rk[i + 2] = rk[i - 2] ^ rk[i + 1];
-        rk[i + 3] = rk[i - 1] ^ rk[i + 2];
+        b ^= a;
+        c ^= b;
+        d ^= c;
+        rk[i] = a;
+        rk[i + 1] = b;
+        rk[i + 2] = c;
+        rk[i + 3] = d;
     }
 }
 

@@ -192,26 +192,24 @@ __device__ __forceinline__ uint32_t claim(uint32_t* counter, bool need, uint32_t
     return base + __popc(m & ((1u << lane) - 1u));
 }
 
-// Per-trial PRP key schedule (cuckoo_bench.cu:226-232): the "KEY1" block of
-// the trial's offset under the batch key, expanded into gh->rk.
-__device__ __forceinline__ void trial_key(const Lanes& L, const Job& J, GroupHeader* gh) {
+// A trial's seeds from its offset's two blocks under the batch key, by lanes 0
+// and 1 of a warp side by side: the "KEY1" block, expanded into the PRP key
+// schedule gh->rk (cuckoo_bench.cu:226-232), and the "WALK" block, which gives
+// walk seed and affine input map (cuckoo_bench.cu:233-238).
+__device__ __forceinline__ void trial_seeds(const Lanes& L, const Job& J, GroupHeader* gh, uint32_t lane) {
     uint32_t w[4];
-    encrypt_full(L, J.batch_rk, 0x4b455931u, 0, gh->offset, 0x50525031u, w);
-    expand_key(L, w[0], w[1], w[2], w[3], gh->rk);
-}
-
-// Per-trial walk seed and affine input map (cuckoo_bench.cu:233-238): the
-// "WALK" block of the trial's offset under the batch key.
-__device__ __forceinline__ void trial_walk_seed(const Lanes& L, const Job& J, GroupHeader* gh) {
-    uint32_t w[4];
-    encrypt_full(L, J.batch_rk, 0x57414c4bu, 0, gh->offset, 0x524e4731u, w);
-    uint64_t walk = ((uint64_t)w[0] << 32) | w[1];
-    const uint64_t shift = (((uint64_t)w[2] << 32) | w[3]) & J.range_mask;
-    uint64_t input_state = shift ^ 0xd1b54a32d192ed03ULL;
-    gh->step = (splitmix(input_state) | 1ULL) & J.range_mask;
-    gh->shift = shift;
-    gh->rnd = splitmix(walk);
-    gh->walk = walk;
+    encrypt_full(L, J.batch_rk, lane ? 0x57414c4bu : 0x4b455931u, 0, gh->offset, lane ? 0x524e4731u : 0x50525031u, w);
+    if (lane == 0) {
+        expand_key(L, w[0], w[1], w[2], w[3], gh->rk);
+    } else {
+        uint64_t walk = ((uint64_t)w[0] << 32) | w[1];
+        const uint64_t shift = (((uint64_t)w[2] << 32) | w[3]) & J.range_mask;
+        uint64_t input_state = shift ^ 0xd1b54a32d192ed03ULL;
+        gh->step = (splitmix(input_state) | 1ULL) & J.range_mask;
+        gh->shift = shift;
+        gh->rnd = splitmix(walk);
+        gh->walk = walk;
+    }
 }
 
 // Round-1 constants of Feistel round r (r < 8) into the trial's header.
@@ -547,10 +545,8 @@ __device__ __forceinline__ void producer(const EngineArgs& a, char* smem, CtaSha
         group_sync(g, gthreads);
         const Job& J = gh->jd;
 
-        // Per-trial PRP key and walk seed (cuckoo_bench.cu:226-238).
+        if (gt < 2) trial_seeds(L, J, gh, gt);
         if (gt == 0) {
-            trial_key(L, J, gh);
-            trial_walk_seed(L, J, gh);
             gh->cand_next = 0;
             // Claim a free slot (FREE -> FILLING).  In-CTA slots: any free
             // one, starting from this group's share of the pool.  Split
@@ -827,11 +823,8 @@ __device__ __forceinline__ void producer_pooled(const EngineArgs& a, char* smem,
                 }
                 __syncwarp();
                 const Job& J = gh->jd;
-                // per-trial PRP key (lane 0) and walk seed (lane 1)
-                if (lane == 0) {
-                    trial_key(L, J, gh);
-                } else if (lane == 1) {
-                    trial_walk_seed(L, J, gh);
+                if (lane < 2) trial_seeds(L, J, gh, lane);
+                if (lane == 2) {
                     gh->cand_next = 0;
                     gh->done = 0;
                 }
