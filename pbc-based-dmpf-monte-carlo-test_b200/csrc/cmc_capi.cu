@@ -237,9 +237,9 @@ int Ctx::plan(const std::vector<Job>& jobs, Plan& pl) {
         };
         if (any_cache ? avg_probe_work >= 512 : avg_probe_work >= 1500) {
             uint32_t most = 0;
-            for (uint32_t ng : {2u, 3u, 4u, 6u}) {
+            for (uint32_t ng : {1u, 2u, 3u, 4u, 6u}) {
                 const uint32_t s = slots_at(ng, pl.group_bytes);
-                if (any_cache && s > most) {
+                if (any_cache && s > most && ng <= std::max(1.0, per_sm + 0.5)) {
                     most = s;
                     cap_ng = ng;
                     pl.wg = 12 / ng;
@@ -250,9 +250,12 @@ int Ctx::plan(const std::vector<Job>& jobs, Plan& pl) {
                 const uint32_t ng = std::min<uint32_t>(kMaxGroups, 15 / wg);
                 const uint32_t pool = pool_group_bytes(round_up(max_cand * entry, 16),
                                                        max_h <= 10 ? fold_table_bytes(max_h) : 0);
-                if (ng > 1 && ng > 2 * per_sm + 1) continue;
+                // a group per trial, where there are no more (of tables below a
+                // warp's width, whose set-up is most of the work, two)
+                if (ng > 1 && ng > (max_cand < 64 ? 2 * per_sm + 1 : per_sm + 0.5)) continue;
+                const uint32_t enough = std::min({4 * ng, 28u, std::max(ng, uint32_t(per_sm) + 1)});
                 if (wg == 1 && direct_pool && slots_at(ng, pool) < 28 && slots_at(13, pool) < 26) continue;
-                if (!(wg == 1 && direct_pool) && slots_at(ng, pl.group_bytes) < std::min(4 * ng, 28u)) continue;
+                if (!(wg == 1 && direct_pool) && slots_at(ng, pl.group_bytes) < enough) continue;
                 pl.wg = wg;
                 pl.isolate = 0;
                 cap_ng = ng;
@@ -415,15 +418,16 @@ double group_cycles(const std::vector<Job>& jobs, const Plan& g, int sms) {
     for (const Job& j : jobs) {
         const double n = j.count, cand = double(j.pnum) * j.k * walk_factor(j);
         const double build = j.method == kMethodDirect ? 8.0 * cand : 8.0 * std::ldexp(1.0, int(j.half_bits));
-        const double rate = wide_domain ? 0.135 : g.pool_stage ? 0.21 : g.slots_smem ? 0.19
-                            : j.method == kMethodCache ? 0.19 : j.method == kMethodGCache ? 0.15 : 0.125;
+        const double rate = wide_domain ? 0.135 : g.pool_stage ? 0.21
+                            : j.method == kMethodGCache ? (g.slots_smem ? 0.17 : 0.15)
+                            : g.slots_smem || j.method == kMethodCache ? 0.19 : 0.125;
         const double lookups = j.method == kMethodCache ? cand : j.method == kMethodGCache ? 1.5 * cand : 0.0;
         trials += n;
         produce += n * ((2.0 + build) / rate + lookups +
                         (g.pool_stage ? 600.0 : (wide_domain ? 25000.0 : 17000.0) / g.ng));
         const double probe = g.slots_smem ? (g.isolate ? (j.mode == CMC_MODE_BGH25 ? 350.0 : 900.0) : 500.0) : 3500.0;
         walk += n * expected_probes(j) * probe / std::max(1u, g.ns);
-        latency = std::max(latency, (expected_probes(j) + straggler_probes(j)) * (g.slots_smem ? 180.0 : 2000.0) +
+        latency = std::max(latency, (expected_probes(j) + straggler_probes(j)) * (g.slots_smem ? 180.0 : 1600.0) +
                                         6.0 * build);
     }
     return std::max(produce, walk) / trials * (trials / sms + 0.5) + latency + 24000.0;
@@ -550,7 +554,7 @@ WavePlan Ctx::plan_waves(const std::vector<Job>& jobs, const Plan& group) const 
 
 // Which engine runs a launch whose group-engine plan is `group`: lanes and
 // waves are left empty where it is the group engine.  The others have to be
-// estimated 8-10 % shorter.
+// estimated 10 and 16 % shorter, about the estimates' error.
 void Ctx::choose_engine(const std::vector<Job>& jobs, const Plan& group, LanePlan& lanes, WavePlan& waves) const {
     lanes = LanePlan{};
     waves = WavePlan{};
@@ -576,7 +580,7 @@ void Ctx::choose_engine(const std::vector<Job>& jobs, const Plan& group, LanePla
     if (force_waves < 0) waves = plan_waves(jobs, group);
     if (force_lanes < 0 && count >= 16ull * sms) lanes = plan_lanes(jobs, group);
     if (!lanes.warps || lanes.cycles >= 0.9 * limit) lanes = LanePlan{};
-    if (!waves.ng || waves.cycles >= 0.92 * limit || (lanes.warps && lanes.cycles < waves.cycles)) waves = WavePlan{};
+    if (!waves.ng || waves.cycles >= 0.84 * limit || (lanes.warps && lanes.cycles < waves.cycles)) waves = WavePlan{};
     if (waves.ng) lanes = LanePlan{};
 }
 
