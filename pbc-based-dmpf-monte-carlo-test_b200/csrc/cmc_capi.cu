@@ -239,7 +239,7 @@ int Ctx::plan(const std::vector<Job>& jobs, Plan& pl) {
             uint32_t most = 0;
             for (uint32_t ng : {1u, 2u, 3u, 4u, 6u}) {
                 const uint32_t s = slots_at(ng, pl.group_bytes);
-                if (any_cache && s > most && ng <= std::max(1.0, per_sm + 0.5)) {
+                if (any_cache && s > most && ng <= std::max(1.0, std::ceil(per_sm))) {
                     most = s;
                     cap_ng = ng;
                     pl.wg = 12 / ng;
@@ -331,7 +331,8 @@ int Ctx::plan(const std::vector<Job>& jobs, Plan& pl) {
         // slots give 3.74 ms and 128 global ones 5.17)
         const double walk_global = ns_g / (probes * (short_launch ? 4500.0 : 3000.0));
         const bool keep_smem = pl.slots_smem && (!may_allocate || walk_smem >= 1.4 * produce ||
-                                                 walk_smem >= walk_global);
+                                                 walk_smem >= walk_global ||
+                                                 (short_launch && !any_gcache && pl.ns > per_sm));  // a slot for every trial
         if (!keep_smem) {
             pl.slots_smem = false;
             pl.nw = nw_g;
