@@ -152,7 +152,7 @@ int Ctx::make_job(const cmc_params& p, uint32_t first, uint32_t count, uint64_t 
 
 // Choose groups, warps per group and slot placement for a set of jobs.
 int Ctx::plan(const std::vector<Job>& jobs, Plan& pl) {
-    uint32_t max_b = 0, max_cand = 0, max_cache_h = 0, any_cache = 0, wide = 0, wide_domain = 0;
+    uint32_t max_b = 0, max_t = 0, max_cand = 0, max_cache_h = 0, any_cache = 0, wide = 0, wide_domain = 0;
     uint32_t max_gcache_h = 0, any_gcache = 0, max_h = 0, dfold_h = 0, any_dfold = 0;
     double work = 0, cand_work = 0;
     for (const Job& j : jobs) {
@@ -162,6 +162,7 @@ int Ctx::plan(const std::vector<Job>& jobs, Plan& pl) {
             dfold_h = std::max(dfold_h, j.half_bits);
         }
         max_b = std::max(max_b, j.buckets);
+        max_t = std::max(max_t, j.pnum);
         max_cand = std::max(max_cand, j.pnum * j.k);
         if (j.method == kMethodCache) {
             any_cache = 1;
@@ -341,6 +342,16 @@ int Ctx::plan(const std::vector<Job>& jobs, Plan& pl) {
         }
     }
     if (!pl.slots_smem) pl.pool_stage = pl.pool_fold = 0;
+    if (!pl.slots_smem && !wide && !pl.walker_ctas) {
+        // global slots of items (item_slots in cmc_engine.cu): [B x 8 bytes]
+        // [t x 8 bytes], as many as the caller's budget
+        // holds beside the round caches
+        pl.bins_bytes = round_up(max_b * 8, 16);
+        pl.slot_stride = round_up(pl.bins_bytes + max_t * 8, 128);
+        const uint64_t caches = any_gcache ? uint64_t(sms) * pl.ng * (16u << max_gcache_h) : 0;
+        const uint64_t fit = (slot_budget - std::min(slot_budget, caches)) / (uint64_t(sms) * pl.slot_stride);
+        if (pl.ns > fit) pl.ns = std::max<uint32_t>(1, uint32_t(fit) / pl.ng) * pl.ng;
+    }
     pl.group_off = kEngineTableBytes + kCtaSharedBytes;
     pl.slots_off = pl.group_off + pl.ng * pl.group_bytes;
     pl.smem_bytes = pl.slots_off + (pl.slots_smem ? pl.ns * pl.slot_stride : 0);

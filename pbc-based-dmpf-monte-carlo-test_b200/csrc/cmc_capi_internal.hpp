@@ -136,6 +136,7 @@ struct Ctx {
     int force_waves = -1;   // wave engine: -1 auto, 0 off, N groups per CTA
     int force_pool = -1;    // pooled direct passes: -1 auto, 0 off, 1 on where they apply
     bool plan_no_dfold = false;  // plan() re-run without room for direct passes' fold tables
+    uint64_t slot_budget = ~0ull;  // bytes for global walk slots and round caches (a server's budget)
     bool group_only = false;   // the caller has no lane or wave engine (a server's launches)
     bool may_allocate = true;  // false: no global round cache, global slots only if unavoidable
     uint32_t spin_limit = 1u << 26;

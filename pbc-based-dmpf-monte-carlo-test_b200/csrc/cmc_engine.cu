@@ -28,15 +28,13 @@
 
 #include "cmc_aes.cuh"
 #include "cmc_engine.cuh"
+#include "cmc_trial.cuh"
 
 namespace cmc {
 
 namespace {
 
-constexpr unsigned kFull = 0xffffffffu;
-constexpr uint32_t kErrBase = 3;     // == -CMC_EKAT: table_base_ok() failed
 constexpr uint32_t kErrTimeout = 4;  // == -CMC_ETIMEOUT
-constexpr uint32_t kErrRange = 5;    // == -CMC_ERANGE
 
 struct GroupHeader {
     unsigned long long gidx;
@@ -144,24 +142,6 @@ __device__ __forceinline__ void group_sync(uint32_t g, uint32_t nthreads) {
     asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "r"(nthreads) : "memory");
 }
 
-__device__ __forceinline__ uint64_t splitmix(uint64_t& s) {
-    s += 0x9E3779B97F4A7C15ULL;
-    uint64_t z = s;
-    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ULL;
-    z = (z ^ (z >> 27)) * 0x94D049BB133111EBULL;
-    return z ^ (z >> 31);
-}
-
-// floor(y / width) for y < 2^32 with magic = floor((2^32 - 1) / width):
-// the estimate is at most two below the quotient and never above it.
-__device__ __forceinline__ uint32_t div_width(uint32_t y, uint32_t width, uint32_t magic) {
-    uint32_t q = __umulhi(y, magic);
-    uint32_t r = y - q * width;
-    if (r >= width) { ++q; r -= width; }
-    if (r >= width) { ++q; }
-    return q;
-}
-
 // c / k for the copy counts k = 2, 3, 4: 0xAAAAAAAB = ceil(2^33 / 3) with a
 // shift of 33 divides every 32-bit c by 3 exactly; 2 and 4 are shifts.
 __device__ __forceinline__ uint32_t div_k(uint32_t c, uint32_t k) {
@@ -219,14 +199,28 @@ __device__ __forceinline__ void store_round1(const Lanes& L, GroupHeader* gh, ui
     gh->r1[r][3] = c.c2; gh->r1[r][4] = c.c3;
 }
 
+// Global walk slots of 16-bit tables hold items with their buckets (ItemWalk in
+// cmc_trial.cuh): [B 8-byte entries][t items' buckets, 8 bytes each].
+template <typename MapT, bool SMEMSLOTS, bool SPLIT>
+__host__ __device__ constexpr bool item_slots() {
+    return !SMEMSLOTS && !SPLIT && sizeof(MapT) == 2;
+}
+
 // ---------------------------------------------------------------- producer --
+
+// Position of pair (o, j) in a map: in order, or (ITEMS) four entries per item
+// (Item in cmc_trial.cuh).
+template <bool ITEMS>
+__device__ __forceinline__ uint32_t map_at(uint32_t cand, uint32_t o, uint32_t j) {
+    return ITEMS ? 4 * o + j : cand;
+}
 
 // FOLD: rounds 1-2 of each pass from the trial's round-2 fold table, kept
 // word-split (component c of entry v at fw[c * n + v], n = 8 << yb) so that a
 // warp's loads of one component are conflict-free while a round has at most
 // 32 entries (h <= 13): 111 table lookups and 4 fold loads per block instead
 // of 124 lookups.
-template <typename MapT, bool WIDE, bool FOLD = false>
+template <typename MapT, bool WIDE, bool FOLD, bool ITEMS>
 __device__ __forceinline__ void build_map_direct(const Lanes& L, const Job& J, GroupHeader* gh,
                                                  const PrpKey& key, MapT* map, uint32_t lane,
                                                  const uint32_t* fw = nullptr) {
@@ -234,11 +228,12 @@ __device__ __forceinline__ void build_map_direct(const Lanes& L, const Job& J, G
     const uint64_t mask = J.mask, domain = J.domain;
     const bool sequential = J.input_mode == 0;
     const uint64_t shift = gh->shift, step = gh->step, range_mask = J.range_mask;
-    uint32_t c = claim(&gh->cand_next, true, lane);
+    uint32_t c = claim(&gh->cand_next, true, lane), at = 0;
     bool has = c < ncand;
     uint64_t left = 0, right = 0;
     auto start = [&](uint32_t cand) {
         const uint32_t o = div_k(cand, k), j = cand - o * k;
+        at = map_at<ITEMS>(cand, o, j);
         const uint64_t e = sequential ? (uint64_t)o : (shift + (uint64_t)o * step) & range_mask;
         const uint64_t y = e * k + j;
         left = y >> h;
@@ -287,7 +282,7 @@ __device__ __forceinline__ void build_map_direct(const Lanes& L, const Job& J, G
             uint32_t b;
             if constexpr (!WIDE) b = div_width((uint32_t)y, (uint32_t)J.width, J.width_magic);
             else b = (uint32_t)(y / J.width);
-            st_map(map + c, b);
+            st_map(map + at, b);
         } else if (has) {
             left = y >> h;
             right = y & mask;
@@ -304,7 +299,7 @@ __device__ __forceinline__ void build_map_direct(const Lanes& L, const Job& J, G
 // Candidates from a round cache (shared or global memory): 8 dependent
 // lookups per Feistel evaluation.  CH independent candidates per lane keep CH
 // lookup chains in flight, which hides the latency of an L2-resident cache.
-template <typename MapT, int CH>
+template <typename MapT, int CH, bool ITEMS>
 __device__ __forceinline__ void build_map_cache(const Job& J, GroupHeader* gh,
                                                 const uint16_t* cache, MapT* map,
                                                 uint32_t lane) {
@@ -313,10 +308,11 @@ __device__ __forceinline__ void build_map_cache(const Job& J, GroupHeader* gh,
     const uint32_t domain_m1 = (uint32_t)(J.domain - 1);
     const bool sequential = J.input_mode == 0;
     const uint64_t shift = gh->shift, step = gh->step, range_mask = J.range_mask;
-    uint32_t c[CH], l[CH], r[CH];
+    uint32_t c[CH], l[CH], r[CH];  // c: the candidate, then its place in the map
     bool has[CH];
     auto start = [&](int i) {
         const uint32_t o = div_k(c[i], k), j = c[i] - o * k;
+        c[i] = map_at<ITEMS>(c[i], o, j);
         const uint64_t e = sequential ? (uint64_t)o : (shift + (uint64_t)o * step) & range_mask;
         const uint32_t y = (uint32_t)(e * k + j);
         l[i] = y >> h;
@@ -364,13 +360,13 @@ __device__ __forceinline__ void build_map_cache(const Job& J, GroupHeader* gh,
     }
 }
 
-template <typename MapT>
+template <typename MapT, bool ITEMS>
 __device__ __forceinline__ void map_from_cache(const Job& J, GroupHeader* gh, const uint16_t* cache,
                                                MapT* map, uint32_t lane, uint32_t chains) {
-    if (chains >= 8) build_map_cache<MapT, 8>(J, gh, cache, map, lane);
-    else if (chains >= 4) build_map_cache<MapT, 4>(J, gh, cache, map, lane);
-    else if (chains == 2) build_map_cache<MapT, 2>(J, gh, cache, map, lane);
-    else build_map_cache<MapT, 1>(J, gh, cache, map, lane);
+    if (chains >= 8) build_map_cache<MapT, 8, ITEMS>(J, gh, cache, map, lane);
+    else if (chains >= 4) build_map_cache<MapT, 4, ITEMS>(J, gh, cache, map, lane);
+    else if (chains == 2) build_map_cache<MapT, 2, ITEMS>(J, gh, cache, map, lane);
+    else build_map_cache<MapT, 1, ITEMS>(J, gh, cache, map, lane);
 }
 
 // Round cache: entry (r, R) = F_r(R) & mask for the 8 rounds and every h-bit
@@ -455,6 +451,7 @@ __device__ __forceinline__ void build_fold_table_split(const Lanes& L, const Prp
 template <typename MapT, typename BinT, bool WIDE, bool SPLIT, bool SMEMSLOTS>
 __device__ __forceinline__ void producer(const EngineArgs& a, char* smem, CtaShared* cs, uint32_t g,
                                          uint32_t gt) {
+    constexpr bool ITEMS = item_slots<MapT, SMEMSLOTS, SPLIT>();
     const uint32_t gthreads = a.wg * 32;
     const uint32_t lane = threadIdx.x & 31;
     const Lanes L{lane * 4, lane * 4 + 128, a.r256};
@@ -623,7 +620,7 @@ __device__ __forceinline__ void producer(const EngineArgs& a, char* smem, CtaSha
         BinT* bins = reinterpret_cast<BinT*>(sbase);
         MapT* map = reinterpret_cast<MapT*>(sbase + a.bins_bytes);
         {
-            const uint32_t nvec = (J.buckets * (uint32_t)sizeof(BinT) + 15) / 16;
+            const uint32_t nvec = (J.buckets * (ITEMS ? 8u : (uint32_t)sizeof(BinT)) + 15) / 16;
             uint4* b4 = reinterpret_cast<uint4*>(bins);
             for (uint32_t i = gt; i < nvec; i += gthreads) b4[i] = make_uint4(kFull, kFull, kFull, kFull);
         }
@@ -632,7 +629,7 @@ __device__ __forceinline__ void producer(const EngineArgs& a, char* smem, CtaSha
             fill_round_cache<SMEMSLOTS, true>(L, key, gh, fold, cache, J.half_bits, (uint32_t)J.mask,
                                               gt, gthreads, a.fill_blocks);
             group_sync(g, gthreads);
-            map_from_cache<MapT>(J, gh, cache, map, lane, a.map_chains ? a.map_chains : 1);
+            map_from_cache<MapT, ITEMS>(J, gh, cache, map, lane, a.map_chains ? a.map_chains : 1);
         } else if (glob_cache) {
             uint16_t* gc = a.gcache + (size_t)(blockIdx.x * a.ng + g) * a.gcache_stride;
             fill_round_cache<SMEMSLOTS, false>(L, key, gh, fold, gc, J.half_bits, (uint32_t)J.mask,
@@ -642,12 +639,12 @@ __device__ __forceinline__ void producer(const EngineArgs& a, char* smem, CtaSha
             // (c = 2^2h / D > 2), where idle chains' gathers cost more than
             // the overlap gains (measured: t=1500, k=4, c~4: 4 chains 8% slower)
             const bool light_walk = (1ULL << (2 * J.half_bits)) <= 2 * J.domain;
-            map_from_cache<MapT>(J, gh, gc, map, lane, a.map_chains ? a.map_chains : (light_walk ? 4 : 2));
+            map_from_cache<MapT, ITEMS>(J, gh, gc, map, lane, a.map_chains ? a.map_chains : (light_walk ? 4 : 2));
         } else if (SMEMSLOTS && !WIDE && direct_fold) {
-            build_map_direct<MapT, WIDE, SMEMSLOTS && !WIDE>(L, J, gh, key, map, lane,
+            build_map_direct<MapT, WIDE, SMEMSLOTS && !WIDE, ITEMS>(L, J, gh, key, map, lane,
                                                              reinterpret_cast<const uint32_t*>(fold));
         } else {
-            build_map_direct<MapT, WIDE>(L, J, gh, key, map, lane);
+            build_map_direct<MapT, WIDE, false, ITEMS>(L, J, gh, key, map, lane);
         }
         if constexpr (SPLIT) __threadfence();
         else __threadfence_block();
@@ -1169,13 +1166,68 @@ struct Walk {
     }
 };
 
+// What the walker loop needs of a walk: one over plain slots, or over items.
+template <typename MapT, typename BinT, bool SMEM>
+struct SlotWalk : Walk<MapT, BinT, SMEM> {
+    __device__ __forceinline__ void run(unsigned long long& probes) {
+        if (this->bgh) {
+            if constexpr (SMEM) {
+                this->top_up();
+                this->bgh_steps(32, probes);
+            } else {
+                this->bgh_steps(64, probes);
+            }
+        } else {
+            this->drrt_steps(64, probes);
+        }
+    }
+};
+
+template <typename BinT>
+struct SlotWalk<uint16_t, BinT, false> : ItemWalk<true> {
+    uint32_t nbins;
+    bool bgh, bad;
+
+    __device__ __forceinline__ void begin(const EngineArgs& a, uint32_t slot, const Job& J, const SlotHeader& h) {
+        char* base = a.gslots + ((size_t)blockIdx.x * a.ns + slot) * a.slot_stride;
+        // at L2: a resident ring entry may have been rewritten since this SM
+        // last read it
+        nbins = __ldcg(&J.buckets);
+        bgh = __ldcg(&J.mode) == 1;
+        bad = false;
+        ItemWalk<true>::begin(base, base + a.bins_bytes, __ldcg(&J.k), __ldcg(&J.pnum), __ldcg(&J.kick), bgh, h.walk,
+                              h.rnd);
+        check();
+    }
+    // A bucket is below B by construction (y < D = B * width); any other value
+    // is recorded as an error instead of being dereferenced.
+    __device__ __forceinline__ void check() {
+        if (bin >= nbins) {
+            bad = failed = true;
+            active = false;
+            bin = 0;
+        }
+    }
+    __device__ __forceinline__ void run(unsigned long long& probes) {
+        uint32_t steps = 0;
+        if (active && bgh) digits.top_up(k);
+#pragma unroll 1
+        for (uint32_t s = 0; s < 16 && active; ++s) {
+            if (bgh) bgh_step(steps);
+            else drrt_step(steps);
+            check();
+        }
+        probes += steps;
+    }
+};
+
 template <typename MapT, typename BinT, bool SMEM>
 __device__ __forceinline__ void walker(const EngineArgs& a, CtaShared* cs, uint32_t wi) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t my = lane * a.nw + wi;  // this lane's slot
     const bool owner = my < a.ns;
-    Walk<MapT, BinT, SMEM> w;
-    w.active = false;
+    SlotWalk<MapT, BinT, SMEM> w;
+    w.active = w.failed = w.bad = false;
     w.bgh = true;
     bool busy = false;  // holds a slot
     unsigned long long gidx = 0;
@@ -1191,15 +1243,7 @@ __device__ __forceinline__ void walker(const EngineArgs& a, CtaShared* cs, uint3
             w.begin(a, my, a.jobs[job], h);
             busy = true;
         }
-        if (w.bgh) {
-            if constexpr (SMEM) {
-                w.top_up();
-                w.bgh_steps(32, probes);
-            } else {
-                w.bgh_steps(64, probes);
-            }
-        }
-        else w.drrt_steps(64, probes);
+        w.run(probes);
         if (busy && !w.active) {
             if (w.bad) {
                 atomicExch(&a.ctrl->error, kErrRange);
@@ -1406,14 +1450,13 @@ __global__ void __launch_bounds__(512, 1) cmc_engine_split(const EngineArgs a) {
                                          threadIdx.x - (warp / a.wg) * a.wg * 32);
 }
 
-// One instantiation per entry width and walk-slot placement.  The walkers'
-// loop over global slots (two dependent L2/DRAM round trips per probe) turned
-// ~4.4x slower when anything changed the register allocation of the kernel
-// around it -- a 3- and 4-block variant of the round-cache fill, one more
-// value held in the walker (measured, on B200; round trips per warp step
-// 5.2k -> 23k cycles) -- so the global-slot kernels are compiled without those
-// and the shared-slot kernels, whose walks are unaffected, keep the
-// fill_blocks choice.
+// One instantiation per entry width and walk-slot placement.  Over global
+// slots, plain ones (32-bit entries; two dependent L2/DRAM round trips per
+// probe) made the walkers' loop ~4.4x slower whenever anything changed the
+// register allocation of the kernel around it, so those kernels keep a plain
+// 2-block fill.  16-bit tables walk items instead (ItemWalk in cmc_trial.cuh),
+// one round trip per probe: t = 8000, N = 2^24, 16,384 trials 55.7 -> 44.2 ms,
+// DRRT18 t = 9707, N = 2^20 102.8 -> 56.8 ms.
 template <typename MapT, typename BinT, bool WIDE, bool SMEMSLOTS>
 __global__ void __launch_bounds__(512, 1) cmc_engine(const EngineArgs a) {
     if (!table_base_ok()) {

@@ -350,7 +350,7 @@ struct Server {
     // Plan for a set of active parameter sets; returns the global pool bytes
     // the plan needs: walk slots (0 for shared-memory slots), then round caches.
     int plan_for(const std::vector<uint32_t>& ids, Plan& pl, std::vector<Job>& shapes, uint64_t& pool,
-                 const std::vector<uint32_t>* weights = nullptr) {
+                 const std::vector<uint32_t>* weights = nullptr, bool for_resident = false) {
         shapes.clear();
         for (size_t i = 0; i < ids.size(); ++i) {
             Job j;
@@ -358,7 +358,11 @@ struct Server {
             if (rc) return fail(rc, ctx->err);
             shapes.push_back(j);
         }
+        // walk slots give way to the budget, of which an iteration gets half
+        ctx->slot_budget = (mem_budget - fixed_bytes) / (for_resident ? 1 : 2);
+        ctx->slot_budget -= std::min<uint64_t>(ctx->slot_budget, 256);  // the caches' alignment
         int rc = ctx->plan(shapes, pl);
+        ctx->slot_budget = ~0ull;
         if (rc) return fail(rc, ctx->err);
         pool = cache_offset(pl) + pl.gcache_bytes;
         return CMC_OK;
@@ -836,7 +840,7 @@ struct Server {
         ctx->force_walkers = 4;
         ctx->force_walker_ctas = 0;
         std::vector<Job> shapes;
-        const int rc = plan_for(ids, pl, shapes, pool);
+        const int rc = plan_for(ids, pl, shapes, pool, nullptr, true);
         ctx->force_global_slots = gs;
         ctx->force_walkers = wk;
         ctx->force_isolate = iso;
@@ -852,8 +856,10 @@ struct Server {
         if (plan_for({id}, one, shapes, pool)) return false;
         const uint32_t entry = r_plan.variant ? 4 : 2;
         const Job& j = shapes[0];
-        const uint64_t bins = (uint64_t(j.buckets) * entry + 15) / 16 * 16;
-        const uint64_t map = (uint64_t(j.pnum) * j.k * entry + 15) / 16 * 16;
+        // slots of items for 16-bit tables (Ctx::plan), else bins and a k-fold map
+        const bool items = r_plan.variant == 0;
+        const uint64_t bins = (uint64_t(j.buckets) * (items ? 8 : entry) + 15) / 16 * 16;
+        const uint64_t map = items ? uint64_t(j.pnum) * 8 : (uint64_t(j.pnum) * j.k * entry + 15) / 16 * 16;
         // the map of every slot starts at the plan's bins_bytes
         return one.variant <= r_plan.variant && bins <= r_plan.bins_bytes &&
                r_plan.bins_bytes + map <= r_plan.slot_stride;

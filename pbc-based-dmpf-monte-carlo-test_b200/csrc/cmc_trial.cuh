@@ -261,6 +261,119 @@ struct Item<false> {
     static __device__ __forceinline__ bool empty(const Entry& e) { return e.w == 0xffffffffu; }
 };
 
+// One trial's walk over a table of entries whose items carry their buckets, a
+// probe per step: one table read, and both of its outcomes (item placed, item
+// evicted) as selects.  A walk alone is bound by latency, the table read and
+// the chain of instructions behind it; beside fills by the ALU pipe, which they
+// use to 85 %.  The walk's digits are therefore decoded ahead, for all lanes
+// together (top_up), and an item that returns to the bin it left costs no read
+// (t = 1024, N = 2^20: 250 ALU instructions per step with 64-bit digit
+// divisions and a loop over returning items; 3,500 cycles a step with 32 lanes
+// and branches).
+template <bool NARROW>
+struct ItemWalk {
+    using ItemT = Item<NARROW>;
+    using Entry = typename ItemT::Entry;
+    Entry* bins;
+    const Entry* map;  // the items' buckets
+    uint32_t k, last, kick;
+    Digits digits;
+    ItemT it;           // the item in hand, number cur, and its copy to try
+    Entry ahead, mine;  // the next item's buckets; what this walk wrote last
+    uint32_t item, cur, count, which, bin;
+    bool again, evicting, active, failed;
+
+    __device__ __forceinline__ void begin(char* table, const char* buckets, uint32_t copies, uint32_t t, uint32_t limit,
+                                          bool bgh, uint64_t walk, uint64_t rnd) {
+        bins = reinterpret_cast<Entry*>(table);
+        map = reinterpret_cast<const Entry*>(buckets);
+        k = copies;
+        last = t - 1;
+        kick = limit;
+        digits = Digits{};
+        digits.walk = walk;
+        digits.rnd = rnd;
+        it = ItemT::from(ItemT::load(map));
+        ahead = ItemT::load(map + 1);  // t >= 3
+        mine = ahead;
+        item = cur = count = 0;
+        again = evicting = failed = false;
+        active = true;
+        which = bgh ? digits.next(k) : 0u;
+        bin = it.get(which);
+    }
+
+    // BGH25 random walk (cuckoo_core.hpp:123-133); an item that returns to the
+    // bin it left finds the item that evicted it, the second time in one step.
+    __device__ __forceinline__ void bgh_step(uint32_t& steps) {
+        const bool four = k == 4;
+        Entry old = mine;
+        if (!again) old = ItemT::load(bins + bin);
+        mine = it.pack(cur, which, four);
+        ++steps;
+        which = digits.next(k);
+        const bool placed = ItemT::empty(old);
+        uint32_t copy;
+        it.unpack(old, bin, four, cur, copy);
+        active = !(placed && item == last);
+        item += placed;
+        it = placed ? ItemT::from(ahead) : it;
+        cur = placed ? item : cur;
+        copy = placed ? 4u : copy;
+        count = placed ? 0u : count + 1;
+        if (placed) ahead = ItemT::load(map + min(item + 1, last));
+        failed = count > kick;
+        if (which == copy && !failed) {
+            ++steps;
+            const Entry back = it.pack(cur, which, four);
+            it.unpack(mine, bin, four, cur, copy);
+            mine = back;
+            which = digits.next(k);
+            failed = ++count > kick;
+        }
+        ItemT::store(bins + bin, mine);
+        active = active && !failed;
+        again = which == copy;
+        bin = it.get(which);
+    }
+
+    // DRRT18 cycling eviction (cuckoo_core.hpp:134-158).
+    __device__ __forceinline__ void drrt_step(uint32_t& steps) {
+        const bool four = k == 4;
+        const Entry old = ItemT::load(bins + bin);
+        const Entry entry = it.pack(cur, which, four);
+        ++steps;
+        const bool placed = ItemT::empty(old), evict = evicting && !placed;
+        if (placed || (evict && count < kick)) ItemT::store(bins + bin, entry);
+        active = !(placed && item == last);
+        item += placed;
+        failed = evict && count >= kick;
+        uint32_t out, copy;  // the item in the bin
+        ItemT there = ItemT::from(old);
+        there.unpack(old, bin, four, out, copy);
+        // an evicted item goes to its next copy in another bin; the copy it sat
+        // by is this bin
+        uint32_t next = copy + 1 == k ? 0 : copy + 1;
+        for (uint32_t tried = 1; evict && there.get(next) == bin; ++tried) {
+            if (tried + 1 == k) {
+                failed = true;
+                break;
+            }
+            next = next + 1 == k ? 0 : next + 1;
+        }
+        // a new item tries its copies in order before it evicts
+        const bool tried_all = !evicting && which + 1 == k;
+        which = placed ? 0u : evict ? next : tried_all ? 0u : which + 1;
+        count = evict ? count + 1 : 0u;
+        it = placed ? ItemT::from(ahead) : evict ? there : it;
+        cur = placed ? item : evict ? out : cur;
+        evicting = !placed && (evicting || tried_all);
+        if (placed) ahead = ItemT::load(map + min(item + 1, last));
+        active = active && !failed;
+        bin = it.get(which);
+    }
+};
+
 // Set-up record of one trial, word w of record e at stock[w * 32 + e].
 enum TrialRecord : uint32_t {
     kStFold = 0,      // narrow: 32 fold words
