@@ -220,27 +220,29 @@ int Ctx::plan(const std::vector<Job>& jobs, Plan& pl) {
     // groups overlap their serial set-ups and barriers.  Measured on B200
     // against three 4-warp groups: t=30, N=2^8 0.121 against 0.211 ms (14 x 1),
     // t=200, N=2^16 0.654 against 0.777 (7 x 2), t=600, N=2^24 1.46 against 1.75
-    // (5 x 3), t=1300 3.01 against 3.47 (3 x 5), t=300, k=4 (h=12) 1.68 against
+    // (5 x 3), t=1300 3.01 against 3.47 (3 x 5),
+    // t=2092, k=2 5.43 against 6.43 (2 x 7), t=300, k=4 (h=12) 1.68 against
     // 1.92 (2 x 7).  Direct passes in pooled one-warp groups only where 13 or 14
     // fit (t=280: 12 pooled groups 0.98 ms, 7 x 2 0.75).  Shared caches with long
     // walks keep the walker isolated and take the split with most slots (t=700,
-    // N=2^16: 21 slots 1.22 ms, 16 slots 1.40).
+    // N=2^16: 21 slots 1.22 ms, 16 slots 1.40).  64-bit domains, whose set-up is
+    // longest, keep their one-warp groups (t=391, k=4: 1.96 against 2.13 ms).
     const double per_sm = work / sms;
     const bool short_launch = !may_allocate || group_only || per_sm <= 200;
     if (short_launch && !force_wg && !force_ng && !force_walkers && force_isolate < 0 &&
-        !pl.walker_ctas && !any_gcache) {
-        const bool direct_pool = force_pool != 0 && !any_cache && !wide_domain;
+        !pl.walker_ctas && !any_gcache && !wide_domain) {
+        const bool direct_pool = force_pool != 0 && !any_cache;
         auto slots_at = [&](uint32_t ng, uint32_t bytes) {
             return ng * bytes > budget
                        ? 0u
                        : ng * std::min<uint32_t>({(budget - ng * bytes) / pl.slot_stride / ng, 32 / ng,
                                                   max_slots_per_group});
         };
-        if (any_cache ? avg_probe_work >= 512 : avg_probe_work >= 1500) {
+        if (any_cache && avg_probe_work >= 512) {
             uint32_t most = 0;
             for (uint32_t ng : {1u, 2u, 3u, 4u, 6u}) {
                 const uint32_t s = slots_at(ng, pl.group_bytes);
-                if (any_cache && s > most && ng <= std::max(1.0, std::ceil(per_sm))) {
+                if (s > most && ng <= std::max(1.0, std::ceil(per_sm))) {
                     most = s;
                     cap_ng = ng;
                     pl.wg = 12 / ng;
@@ -249,12 +251,13 @@ int Ctx::plan(const std::vector<Job>& jobs, Plan& pl) {
         } else {
             for (uint32_t wg : {1u, 2u, 3u, 5u, 7u, 15u}) {
                 const uint32_t ng = std::min<uint32_t>(kMaxGroups, 15 / wg);
+                if (ng == 1 && avg_probe_work >= 1500) break;  // long walks: isolated walkers, global slots
                 const uint32_t pool = pool_group_bytes(round_up(max_cand * entry, 16),
                                                        max_h <= 10 ? fold_table_bytes(max_h) : 0);
                 // a group per trial, where there are no more (of tables below a
                 // warp's width, whose set-up is most of the work, two)
                 if (ng > 1 && ng > (max_cand < 64 ? 2 * per_sm + 1 : per_sm + 0.5)) continue;
-                const uint32_t enough = std::min({4 * ng, 28u, std::max(ng, uint32_t(per_sm) + 1)});
+                const uint32_t enough = std::min({4 * ng, 28u, std::max(2 * ng, uint32_t(per_sm) + 1)});
                 if (wg == 1 && direct_pool && slots_at(ng, pool) < 28 && slots_at(13, pool) < 26) continue;
                 if (!(wg == 1 && direct_pool) && slots_at(ng, pl.group_bytes) < enough) continue;
                 pl.wg = wg;
