@@ -116,6 +116,27 @@ uint32_t choose_method(uint32_t h, uint64_t domain, double candidates, int force
     return kMethodDirect;
 }
 
+// Job::last_rows and last_cuts.  L's above the domain lead to another pass and
+// need their round; of the others a bucket no narrower than 2^h cuts at most
+// one per bucket, at 119 shared-memory wavefronts per 32 entries against 106 in
+// rows.  Rows are dropped in pairs (the fill loops' step), and only where a
+// sixteenth of the fill goes with them (3 % at t = 1500, k = 4, N = 2^24 lost as
+// much in the lookups).  t = 1024, k = 3, N = 2^20 needs 512 of 2048 entries.
+static void last_round(Job& j) {
+    const uint32_t h = j.half_bits;
+    if (j.domain > 0xffffffffULL || h < 9 || h > 16 || j.width < (1ULL << h)) return;
+    const uint32_t rows = uint32_t(j.domain >> h >> 8) & ~1u;
+    const uint64_t cuts = j.width & j.mask ? (j.domain - 1) / j.width : 0;
+    if (256.0 * rows - 1.15 * cuts < j.mask / 2) return;
+    j.last_rows = rows;
+    j.last_cuts = uint32_t(cuts);
+}
+
+// AES blocks of a round cache.
+static double cache_blocks(const Job& j) {
+    return 8.0 * std::ldexp(1.0, int(j.half_bits)) - 256.0 * j.last_rows + 1.15 * j.last_cuts;
+}
+
 // Fill a device job descriptor from derived parameters.
 int Ctx::make_job(const cmc_params& p, uint32_t first, uint32_t count, uint64_t base, Job& j) {
     std::memset(&j, 0, sizeof j);
@@ -147,6 +168,7 @@ int Ctx::make_job(const cmc_params& p, uint32_t first, uint32_t count, uint64_t 
     j.count = count;
     j.trial_base = base;
     j.method = choose_method(p.half_bits, p.domain, double(p.pnum) * p.k, force_method, may_allocate);
+    last_round(j);
     return CMC_OK;
 }
 
@@ -505,8 +527,8 @@ LanePlan Ctx::plan_lanes(const std::vector<Job>& jobs, const Plan& group) const 
 }
 
 // The wave engine's form of a launch (ng == 0: it does not fit).  A map costs
-// the fill (8 * 2^h blocks at 106 wavefronts per 32 and 98 % of the shared-memory
-// pipe: 27.2 cycles * 2^h), its lookups and 3 cycles per probe; a walk step
+// the fill (8 * 2^h blocks or less at 106 wavefronts per 32 and 98 % of the shared-memory
+// pipe: 3.4 cycles a block), its lookups and 3 cycles per probe; a walk step
 // takes 900 cycles and 145 more per lane of the warp.  Fewer groups lose overlap
 // of fill, map and walk; more than two spill global caches out of L2.
 WavePlan Ctx::plan_waves(const std::vector<Job>& jobs, const Plan& group) const {
@@ -520,7 +542,7 @@ WavePlan Ctx::plan_waves(const std::vector<Job>& jobs, const Plan& group) const 
     const bool gc = max_h > 12;
     for (const Job& j : jobs) {
         const double cand = double(j.pnum) * j.k * walk_factor(j);
-        build += j.count * (27.2 * std::ldexp(1.0, int(j.half_bits)) + (gc ? 6.0 : 1.8) * cand +
+        build += j.count * (3.4 * cache_blocks(j) + (gc ? 6.0 : 1.8) * cand +
                             3.0 * expected_probes(j) + 1200.0);
         probes = std::max(probes, expected_probes(j));
         stragglers = std::max(stragglers, straggler_probes(j));

@@ -50,6 +50,12 @@ struct Job {
     uint32_t count;         // trials of this job in the launch
     uint32_t user;          // caller tag (job id in batched/served mode)
     uint64_t trial_base;
+    // The last Feistel round of a round cache (wave engine).  It sets the low half of the PRP
+    // output y = L << h | R, and the bucket y / width often follows from L
+    // alone: its entries for inputs L < 256 * last_rows are needed only where a
+    // bucket begins inside [L << h, (L + 1) << h), at m * width for
+    // m = 1 .. last_cuts.  last_rows == 0: the round is filled and read whole.
+    uint32_t last_rows, last_cuts;
 };
 
 struct Ctrl {

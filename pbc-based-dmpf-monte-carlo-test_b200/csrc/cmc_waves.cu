@@ -61,9 +61,10 @@ __device__ __forceinline__ uint4 wave_u(const Lanes& L, uint32_t c0, uint32_t w)
     return make_uint4(T2::e0<3>(L, a), T2::e3<0>(L, a), T2::e2<1>(L, a), T2::e1<2>(L, a));
 }
 
-// Round cache entries (r << h) | R = F_r(R) & mask.
+// Round cache entries (r << h) | R = F_r(R) & mask; of round 7 those that the
+// buckets need (Job::last_rows; t = 1024, N = 2^20: 9 % of all blocks less).
 template <bool GC>
-__device__ __forceinline__ void wave_fill(const Lanes& L, const PrpKey& key, uint32_t c0, uint32_t k3,
+__device__ __forceinline__ void wave_fill(const Lanes& L, const PrpKey& key, const Job& J, uint32_t c0, uint32_t k3,
                                           uint32_t fold, uint16_t* cache, uint32_t h, uint32_t mask,
                                           uint32_t gt, uint32_t nt) {
     const uint32_t cbase = GC ? 0 : (uint32_t)__cvta_generic_to_shared(cache);
@@ -72,19 +73,36 @@ __device__ __forceinline__ void wave_fill(const Lanes& L, const PrpKey& key, uin
         else st_cache_shared(cbase + 2 * e, v);
     };
     if (h >= 8) {
-        const uint32_t n = 8u << (h - 8);  // (r, y) pairs
-        const uint32_t parts = nt > 256 ? nt / 256 : 1;
-        const uint32_t i0 = (gt >> 8) * (n / parts), i1 = i0 + n / parts;
+        const uint32_t last = 7u << (h - 8), rows = J.last_rows;  // (r, y) pairs of rounds 0..6
+        const uint32_t n = (8u << (h - 8)) - rows;
+        const uint32_t parts = nt > 256 ? nt / 256 : 1, part = gt >> 8;
+        const uint32_t n0 = n * part / parts & ~1u, n1 = part + 1 == parts ? n : n * (part + 1) / parts & ~1u;
+        const uint32_t begin = n0 < last ? n0 : n0 + rows, end = n1 > last ? n1 + rows : n1;
+        const uint32_t mid = rows && begin < last ? min(n1, last) : end;
         for (uint32_t x = gt & 255u; x < 256; x += nt) {
             const uint4 u = wave_u(L, c0, x ^ k3);
+            uint32_t i = begin, stop = mid;
 #pragma unroll 1
-            for (uint32_t i = i0; i < i1; i += 2) {
-                const uint4 f = lds_fold(fold + 16 * i), g = lds_fold(fold + 16 * i + 16);
-                const uint32_t a = prp_tail(L, key, u.x ^ f.x, u.y ^ f.y, u.z ^ f.z, u.w ^ f.w);
-                const uint32_t b = prp_tail(L, key, u.x ^ g.x, u.y ^ g.y, u.z ^ g.z, u.w ^ g.w);
-                put(256 * i + x, a & mask);
-                put(256 * i + 256 + x, b & mask);
+            for (;;) {  // [begin, mid), then [last + rows, end)
+#pragma unroll 1
+                for (; i < stop; i += 2) {
+                    const uint4 f = lds_fold(fold + 16 * i), g = lds_fold(fold + 16 * i + 16);
+                    const uint32_t a = prp_tail(L, key, u.x ^ f.x, u.y ^ f.y, u.z ^ f.z, u.w ^ f.w);
+                    const uint32_t b = prp_tail(L, key, u.x ^ g.x, u.y ^ g.y, u.z ^ g.z, u.w ^ g.w);
+                    put(256 * i + x, a & mask);
+                    put(256 * i + 256 + x, b & mask);
+                }
+                if (stop == end) break;
+                i = last + rows;
+                stop = end;
             }
+        }
+        const uint32_t width = (uint32_t)J.width;
+        for (uint32_t m = gt + 1; m <= J.last_cuts; m += nt) {
+            const uint32_t at = m * width, R = at >> h;
+            if ((at & mask) == 0 || R >= 256 * rows) continue;
+            const uint4 u = wave_u(L, c0, (R & 255u) ^ k3), f = lds_fold(fold + 16 * (last + (R >> 8)));
+            put((7u << h) + R, prp_tail(L, key, u.x ^ f.x, u.y ^ f.y, u.z ^ f.z, u.w ^ f.w) & mask);
         }
     } else {
         for (uint32_t e = gt; e < 8u << h; e += nt) {
@@ -96,14 +114,16 @@ __device__ __forceinline__ void wave_fill(const Lanes& L, const PrpKey& key, uin
 
 // Buckets of all (item, copy) pairs from a round cache, CH lookup chains per
 // lane; a warp runs over its own share of the pairs and a lane takes the next
-// pair when its cycle-walk ends.  Returns false if a bucket was out of range.
-template <int CH, typename MapT>
+// pair when its cycle-walk ends.  PART: the cache may hold a part of round 7
+// (Job::last_rows).  Returns false if a bucket was out of range.
+template <int CH, bool PART, typename MapT>
 __device__ __forceinline__ bool wave_map(const Job& J, const uint32_t* rec, const uint16_t* cache, MapT* map,
                                          uint32_t gwi, uint32_t wg, uint32_t lane) {
     const uint32_t k = J.k, ncand = J.pnum * k, h = J.half_bits, mask = (uint32_t)J.mask;
     const uint32_t domain_m1 = (uint32_t)(J.domain - 1), width = (uint32_t)J.width, magic = J.width_magic;
     const uint32_t nbins = J.buckets;
-    const bool sequential = J.input_mode == 0;
+    const bool sequential = J.input_mode == 0, cuts = J.last_cuts != 0;
+    const uint32_t whole = J.last_rows ? 2 * (uint32_t)(J.domain >> h) : 0;  // high halves inside the domain
     const uint64_t shift = (uint64_t)rec[kStWalk + 4] | ((uint64_t)rec[kStWalk + 5] << 32);
     const uint64_t step = (uint64_t)rec[kStWalk + 6] | ((uint64_t)rec[kStWalk + 7] << 32);
     const uint64_t rmask = J.range_mask;
@@ -138,11 +158,34 @@ __device__ __forceinline__ bool wave_map(const Job& J, const uint32_t* rec, cons
     }
     while (__any_sync(kFull, any)) {
 #pragma unroll
-        for (uint32_t rr = 0; rr < 8; ++rr) {
+        for (uint32_t rr = 0; rr < (PART ? 7 : 8); ++rr) {
             const char* round = reinterpret_cast<const char*>(cache) + ((size_t)rr << (h + 1));
 #pragma unroll
             for (int i = 0; i < CH; ++i) {
                 const uint32_t nr = l[i] ^ 2u * *reinterpret_cast<const uint16_t*>(round + r[i]);
+                l[i] = r[i];
+                r[i] = nr;
+            }
+        }
+        if constexpr (PART) {
+            // The last round, where the bucket does not follow from the high half
+            // (with any low half y is then in the domain and in the same bucket).
+            const char* round = reinterpret_cast<const char*>(cache) + ((size_t)7 << (h + 1));
+            bool decided[CH];
+#pragma unroll
+            for (int i = 0; i < CH; ++i) decided[i] = r[i] < whole;
+            if (cuts) {
+#pragma unroll
+                for (int i = 0; i < CH; ++i) {
+                    const uint32_t y0 = (r[i] >> 1) << h;
+                    decided[i] = decided[i] && (div_width(y0, width, magic) + 1) * width - y0 > mask;
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < CH; ++i) {
+                uint32_t f = 0;
+                if (!decided[i]) f = *reinterpret_cast<const uint16_t*>(round + r[i]);
+                const uint32_t nr = l[i] ^ 2u * f;
                 l[i] = r[i];
                 r[i] = nr;
             }
@@ -378,10 +421,11 @@ __global__ void __launch_bounds__(512, 1) cmc_waves(const WaveArgs a) {
             key.kr[30] = rol8(rec[kStKey + 25]);
             key.k43lo = rec[kStKey + 28] & 0xffffu;
             wave_sync(g, nt);
-            wave_fill<GC>(L, key, rec[kStKey + 26], k3, fold, cache, h, mask, gt, nt);
+            wave_fill<GC>(L, key, J, rec[kStKey + 26], k3, fold, cache, h, mask, gt, nt);
             wave_sync(g, nt);
             MapT* map = reinterpret_cast<MapT*>(region + a.map_off);
-            ok = wave_map<GC ? 4 : 2>(J, rec, cache, map, gt >> 5, a.wg, lane) && ok;
+            ok = (GC || J.last_rows ? wave_map<GC ? 4 : 2, true>(J, rec, cache, map, gt >> 5, a.wg, lane)
+                                    : wave_map<GC ? 4 : 2, false>(J, rec, cache, map, gt >> 5, a.wg, lane)) && ok;
         }
         wave_sync(g, nt);
         auto get64 = [&](uint32_t w) {

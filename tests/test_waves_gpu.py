@@ -77,3 +77,30 @@ def test_waves_job_table(ctx, cmc):
     ctx.set_option("waves", 2)
     assert ctx.run_jobs(jobs) == want
     assert "engine=waves" in ctx.last_plan
+
+
+@pytest.mark.parametrize("groups", [1, 2, 8])
+@pytest.mark.parametrize("shape", [
+    # round 7 filled in part: buckets that end with a high half (no cuts), and
+    # not; domains of 3/4, 3/8 and nearly all of 4^h; each end of the widths
+    ("bgh25", "affine", 64, 20, 3, 96, 20, 1500),          # h = 11, 512 of 2048 entries
+    ("bgh25", "sequential", 64, 20, 3, 75, 30, 1500),      # h = 11, 74 cuts
+    ("drrt18", "affine", 93, 18, 3, 110, 30, 1500),        # h = 10, two rows of four
+    ("bgh25", "affine", 300, 19, 3, 330, 50, 600),         # h = 11, 3/8, most fail
+    ("bgh25", "affine", 50, 21, 2, 113, 10, 1500),         # h = 11, one entry above 4^h / 2
+    ("drrt18", "sequential", 40, 22, 4, 4096, 3, 500),     # h = 12, the whole of 4^h
+    ("bgh25", "affine", 1000, 24, 3, 1100, 60, 200),       # h = 13, global cache
+    ("drrt18", "affine", 150, 30, 3, 170, 60, 100),        # h = 16
+])
+def test_part_of_last_round(ctx, cmc, oracle, shape, groups):
+    mode, im, t, ell, k, buckets, kick, n = shape
+    p = cmc.parameters(mode, t, ell, k, buckets, kick, im)
+    want = oracle.batch(oracle.params(mode, t, ell, k, buckets, kick, im), 5, 1, 3, n)
+    ctx.set_option("waves", groups)
+    assert ctx.launch(p, cmc.batch_key(5, 1), 3, n) == want
+    assert "engine=waves" in ctx.last_plan
+    probes = ctx.last_stats()["probes"]
+    ctx.set_option("waves", 0)
+    ctx.set_option("lanes", 0)
+    assert ctx.launch(p, cmc.batch_key(5, 1), 3, n) == want
+    assert probes == ctx.last_stats()["probes"]
