@@ -530,7 +530,8 @@ LanePlan Ctx::plan_lanes(const std::vector<Job>& jobs, const Plan& group) const 
 // the fill (8 * 2^h blocks or less at 106 wavefronts per 32 and 98 % of the shared-memory
 // pipe: 3.4 cycles a block), its lookups and 3 cycles per probe; a walk step
 // takes 900 cycles and 145 more per lane of the warp.  Fewer groups lose overlap
-// of fill, map and walk; more than two spill global caches out of L2.
+// of fill, map and walk; more than two spill global caches out of L2.  With one
+// group at h = 13, 1.15 is where its lookups begin to pay (about 8,000 passes).
 WavePlan Ctx::plan_waves(const std::vector<Job>& jobs, const Plan& group) const {
     WavePlan wp;
     wp.cycles = 1e300;
@@ -539,38 +540,45 @@ WavePlan Ctx::plan_waves(const std::vector<Job>& jobs, const Plan& group) const 
     uint64_t max_b = 0, max_t = 0;
     uint32_t max_h = 0;
     for (const Job& j : jobs) max_h = std::max(max_h, j.half_bits);
-    const bool gc = max_h > 12;
+    double lookups = 0;
     for (const Job& j : jobs) {
-        const double cand = double(j.pnum) * j.k * walk_factor(j);
-        build += j.count * (3.4 * cache_blocks(j) + (gc ? 6.0 : 1.8) * cand +
-                            3.0 * expected_probes(j) + 1200.0);
+        lookups += j.count * double(j.pnum) * j.k * walk_factor(j);
+        build += j.count * (3.4 * cache_blocks(j) + 3.0 * expected_probes(j) + 1200.0);
         probes = std::max(probes, expected_probes(j));
         stragglers = std::max(stragglers, straggler_probes(j));
         trials += j.count;
         max_b = std::max<uint64_t>(max_b, j.buckets);
         max_t = std::max<uint64_t>(max_t, j.pnum);
     }
-    build /= trials;
     const uint64_t entry = group.variant == 0 ? 8 : 16;
     WavePlan q;
     q.variant = group.variant;
     q.ctas = sms;
-    q.global_cache = gc;
     q.cache_off = kWaveHeaderBytes + fold_table_bytes(max_h);
-    q.group_bytes = q.cache_off + (gc ? 0 : 16u << max_h);
     q.map_off = uint32_t((max_b * entry + 15) / 16 * 16);
     q.region_bytes = (q.map_off + max_t * entry + 127) / 128 * 128;
-    q.gcache_stride = gc ? 8u << max_h : 0;
     for (uint32_t ng : {1u, 2u, 4u, 8u}) {
         if (force_waves > 0 && ng > uint32_t(force_waves)) break;
+        // A round cache of h = 13 (128 KiB) fits in shared memory beside the
+        // T-table for one group.  Its fill and map then no longer overlap, but
+        // the map's gathers from L2 go: one group against two with global
+        // caches 7.2 against 7.4 ms (t=2570, k=3), 40.6 against 43.9 (t=4599,
+        // k=2, 30,000 trials), 23.4 against 26.5 (DRRT18 t=15580).  Parts of
+        // larger caches there measured slower (h=14, 2 of 8 rounds: 47.2 ->
+        // 56.3 ms): L1 holds as much of them and loses that room.
+        const bool gc = max_h > (ng == 1 ? 13 : 12);
+        const double map = (build + (gc ? 6.0 : 1.8) * lookups) / trials;
+        q.global_cache = gc;
+        q.gcache_stride = gc ? 8u << max_h : 0;
+        q.group_bytes = q.cache_off + (gc ? 0 : 16u << max_h);
         q.smem_bytes = kEngineTableBytes + ng * q.group_bytes;
-        if (q.smem_bytes > smem_optin) break;
+        if (q.smem_bytes > smem_optin) continue;
         q.ng = ng;
         q.wg = 16 / ng;
         q.gcache_bytes = uint64_t(sms) * ng * q.gcache_stride * 2;
         const double lost = gc ? (ng == 1 ? 1.02 : ng == 2 ? 1.0 : ng == 4 ? 1.03 : 1.2) *
                                      (q.gcache_bytes > 140000000 ? 1.08 : 1.0)
-                               : (ng == 1 ? 1.3 : ng == 2 ? 1.12 : ng == 4 ? 1.0 : 0.97);
+                               : (ng == 1 ? (max_h == 13 ? 1.15 : 1.3) : ng == 2 ? 1.12 : ng == 4 ? 1.0 : 0.97);
         // One wave where a group's share of the launch fits its threads: the
         // walks of all groups then run once, after all maps.  Longer launches
         // run in waves of equal size; towards the end they shrink to the trials
@@ -578,8 +586,8 @@ WavePlan Ctx::plan_waves(const std::vector<Job>& jobs, const Plan& group) const 
         const double share = std::ceil(trials / (double(sms) * ng)), nt = q.wg * 32, waves = std::ceil(share / nt);
         q.wave = uint32_t(std::ceil(share / waves));
         const double walk = probes * (900.0 + 145.0 * q.wave / q.wg) + 1000.0 * stragglers;
-        q.min_wave = waves > 1 ? uint32_t(std::min(double(q.wave), std::max(1.0, walk / (build * ng)))) : q.wave;
-        const double maps = share * ng * build * lost;
+        q.min_wave = waves > 1 ? uint32_t(std::min(double(q.wave), std::max(1.0, walk / (map * ng)))) : q.wave;
+        const double maps = share * ng * map * lost;
         q.cycles = (waves > 1 ? std::max(maps, waves * walk) : maps) + walk + 60000.0;
         q.regions_bytes = q.region_bytes * sms * ng * q.wave;
         q.stock_bytes = uint64_t(sms) * ng * q.wg * kRecordBlockBytes;

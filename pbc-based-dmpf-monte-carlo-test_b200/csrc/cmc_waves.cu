@@ -334,7 +334,8 @@ __device__ __forceinline__ bool walk_drrt(const Job& J, bool active, char* regio
 }  // namespace
 
 // NARROW: 8-byte table entries, else 16-byte ones (Item in cmc_trial.cuh).  GC:
-// round caches in global memory (h <= 16), else in shared memory (h <= 12).
+// round caches in global memory (h <= 16), else in shared memory (h <= 12, or a
+// single group's of h = 13).
 template <bool NARROW, bool GC>
 __global__ void __launch_bounds__(512, 1) cmc_waves(const WaveArgs a) {
     if (!table_base_ok()) {

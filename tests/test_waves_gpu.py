@@ -104,3 +104,27 @@ def test_part_of_last_round(ctx, cmc, oracle, shape, groups):
     ctx.set_option("lanes", 0)
     assert ctx.launch(p, cmc.batch_key(5, 1), 3, n) == want
     assert probes == ctx.last_stats()["probes"]
+
+
+@pytest.mark.parametrize("shape,groups", [
+    # a round cache of h = 13 in the shared memory of a single group
+    (("bgh25", "affine", 1000, 24, 3, 1100, 60, 200), 1),
+    (("drrt18", "sequential", 333, 24, 2, 800, 40, 300), 1),
+    (("bgh25", "affine", 2000, 22, 4, 2300, 60, 150), 1),    # h = 13, every pair cycle-walks
+    (("drrt18", "affine", 17500, 24, 3, 66000, 60, 16), 1),  # with 32-bit entries
+    # the same width with more groups, and the next width, in global memory
+    (("bgh25", "affine", 1000, 24, 3, 1100, 60, 200), 2),
+    (("bgh25", "affine", 1366, 26, 3, 1500, 60, 100), 1),
+])
+def test_round_cache_places(ctx, cmc, oracle, shape, groups):
+    mode, im, t, ell, k, buckets, kick, n = shape
+    p = cmc.parameters(mode, t, ell, k, buckets, kick, im)
+    want = oracle.batch(oracle.params(mode, t, ell, k, buckets, kick, im), 7, 1, 9, n)
+    ctx.set_option("waves", groups)
+    assert ctx.launch(p, cmc.batch_key(7, 1), 9, n) == want
+    assert "cache=" + ("smem" if p.half_bits == 13 and groups == 1 else "global") in ctx.last_plan.split("->")[-1]
+    probes = ctx.last_stats()["probes"]
+    ctx.set_option("waves", 0)
+    ctx.set_option("lanes", 0)
+    assert ctx.launch(p, cmc.batch_key(7, 1), 9, n) == want
+    assert probes == ctx.last_stats()["probes"]
