@@ -530,7 +530,9 @@ LanePlan Ctx::plan_lanes(const std::vector<Job>& jobs, const Plan& group) const 
 // the fill (8 * 2^h blocks or less at 106 wavefronts per 32 and 98 % of the shared-memory
 // pipe: 3.4 cycles a block), its lookups and 3 cycles per probe; a walk step
 // takes 900 cycles and 145 more per lane of the warp.  Fewer groups lose overlap
-// of fill, map and walk; more than two spill global caches out of L2.  With one
+// of fill, map and walk; more than two spill global caches out of L2, and at
+// h = 16 two do out of L1 (t=12000, k=4, N=2^28: 28.0 ms with one, 34.5 with two;
+// t=4139 48.6 and 51.3).  With one
 // group at h = 13, 1.15 is where its lookups begin to pay (about 8,000 passes).
 WavePlan Ctx::plan_waves(const std::vector<Job>& jobs, const Plan& group) const {
     WavePlan wp;
@@ -576,7 +578,7 @@ WavePlan Ctx::plan_waves(const std::vector<Job>& jobs, const Plan& group) const 
         q.ng = ng;
         q.wg = 16 / ng;
         q.gcache_bytes = uint64_t(sms) * ng * q.gcache_stride * 2;
-        const double lost = gc ? (ng == 1 ? 1.02 : ng == 2 ? 1.0 : ng == 4 ? 1.03 : 1.2) *
+        const double lost = gc ? (ng == 1 ? (max_h == 16 ? 0.95 : 1.02) : ng == 2 ? 1.0 : ng == 4 ? 1.03 : 1.2) *
                                      (q.gcache_bytes > 140000000 ? 1.08 : 1.0)
                                : (ng == 1 ? (max_h == 13 ? 1.15 : 1.3) : ng == 2 ? 1.12 : ng == 4 ? 1.0 : 0.97);
         // One wave where a group's share of the launch fits its threads: the

@@ -425,8 +425,18 @@ __global__ void __launch_bounds__(512, 1) cmc_waves(const WaveArgs a) {
             wave_fill<GC>(L, key, J, rec[kStKey + 26], k3, fold, cache, h, mask, gt, nt);
             wave_sync(g, nt);
             MapT* map = reinterpret_cast<MapT*>(region + a.map_off);
-            ok = (GC || J.last_rows ? wave_map<GC ? 4 : 2, true>(J, rec, cache, map, gt >> 5, a.wg, lane)
-                                    : wave_map<GC ? 4 : 2, false>(J, rec, cache, map, gt >> 5, a.wg, lane)) && ok;
+            // Four chains per lane hide a gather's latency from L2.  Where L1
+            // holds much of the caches (256 KiB at h = 14; a single group's) two
+            // are faster, as the warps' rounds, 2^(h+1) bytes each, stay closer
+            // together: t=1500, k=4 (h = 14) 47.0 -> 44.7 ms, t=4139 (h = 16) in
+            // one group 58.2 -> 48.6, in two 51.4 -> 56.4.
+            if constexpr (GC) {
+                ok = (h > 14 && a.ng > 1 ? wave_map<4, true>(J, rec, cache, map, gt >> 5, a.wg, lane)
+                                         : wave_map<2, true>(J, rec, cache, map, gt >> 5, a.wg, lane)) && ok;
+            } else {
+                ok = (J.last_rows ? wave_map<2, true>(J, rec, cache, map, gt >> 5, a.wg, lane)
+                                  : wave_map<2, false>(J, rec, cache, map, gt >> 5, a.wg, lane)) && ok;
+            }
         }
         wave_sync(g, nt);
         auto get64 = [&](uint32_t w) {

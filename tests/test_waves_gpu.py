@@ -115,6 +115,10 @@ def test_part_of_last_round(ctx, cmc, oracle, shape, groups):
     # the same width with more groups, and the next width, in global memory
     (("bgh25", "affine", 1000, 24, 3, 1100, 60, 200), 2),
     (("bgh25", "affine", 1366, 26, 3, 1500, 60, 100), 1),
+    # global caches with two and with four lookup chains per lane
+    (("drrt18", "affine", 900, 26, 3, 1000, 60, 100), 2),    # h = 14
+    (("bgh25", "affine", 900, 28, 3, 1000, 60, 100), 2),     # h = 15
+    (("bgh25", "affine", 37, 30, 3, 43, 30, 60), 4),         # h = 16, fewer pairs than lanes
 ])
 def test_round_cache_places(ctx, cmc, oracle, shape, groups):
     mode, im, t, ell, k, buckets, kick, n = shape
