@@ -204,6 +204,9 @@ int Ctx::plan(const std::vector<Job>& jobs, Plan& pl) {
     if (wide_domain) wide = 1;
     pl.variant = wide_domain ? 2 : (wide ? 1 : 0);
     const uint32_t entry = wide ? 4 : 2;
+    // slots are addressed by 32-bit offsets
+    if ((uint64_t(max_b) + max_cand) * entry > 0xffffff00ULL)
+        return fail(CMC_EINVAL, "a table of %u buckets exceeds the 4 GiB of a walk slot", max_b);
     pl.bins_bytes = round_up(max_b * entry, 16);
     const uint32_t map_bytes = round_up(max_cand * entry, 16);
     pl.slot_stride = round_up(pl.bins_bytes + map_bytes, 128);
@@ -517,6 +520,7 @@ LanePlan Ctx::plan_lanes(const std::vector<Job>& jobs, const Plan& group) const 
     lp.ctas = sms;
     lp.share = uint32_t(std::min(32.0, std::max(1.0, std::ceil(per_sm / warps))));
     lp.region_bytes = (uint64_t(max_b) * (group.variant == 0 ? 8 : 16) + 127) / 128 * 128;
+    if (lp.region_bytes > 0xffffffffULL) return lp;  // a table is filled by 32-bit counts
     lp.smem_bytes = kLaneTableBytes + warps * kLaneFoldBytes;
     lp.regions_bytes = lp.region_bytes * sms * warps * lp.share;
     lp.stock_bytes = uint64_t(sms) * warps * kRecordBlockBytes;
@@ -557,8 +561,10 @@ WavePlan Ctx::plan_waves(const std::vector<Job>& jobs, const Plan& group) const 
     q.variant = group.variant;
     q.ctas = sms;
     q.cache_off = kWaveHeaderBytes + fold_table_bytes(max_h);
-    q.map_off = uint32_t((max_b * entry + 15) / 16 * 16);
-    q.region_bytes = (q.map_off + max_t * entry + 127) / 128 * 128;
+    const uint64_t map_off = (max_b * entry + 15) / 16 * 16;
+    if (map_off > 0xffffffffULL) return wp;  // WavePlan::map_off
+    q.map_off = uint32_t(map_off);
+    q.region_bytes = (map_off + max_t * entry + 127) / 128 * 128;
     for (uint32_t ng : {1u, 2u, 4u, 8u}) {
         if (force_waves > 0 && ng > uint32_t(force_waves)) break;
         // A round cache of h = 13 (128 KiB) fits in shared memory beside the
