@@ -82,19 +82,57 @@ int Ctx::cuda(cudaError_t e, const char* what) {
     return fail(CMC_ECUDA, "%s: %s", what, cudaGetErrorString(e));
 }
 
-template <typename T>
-int Ctx::grow(T*& ptr, size_t& cap, size_t need, const char* what) {
+// Room for `need` elements of `size` bytes in a device buffer.  A buffer is
+// replaced only by a larger one: the new one is allocated first, and only where
+// both do not fit the old one is given up for it.  During a stream capture
+// (fixed_memory) nothing is allocated or freed: both calls would end the capture.
+int Ctx::grow_bytes(void*& ptr, size_t& cap, size_t need, size_t size, const char* what) {
     if (need <= cap && ptr) return CMC_OK;
-    if (ptr) cudaFree(ptr);
-    ptr = nullptr;
-    cap = 0;
-    size_t n = std::max<size_t>(need, 1);
-    if (cudaMalloc(reinterpret_cast<void**>(&ptr), n * sizeof(T)) != cudaSuccess) {
-        cudaGetLastError();
-        return fail(CMC_ENOMEM, "cudaMalloc of %zu bytes for %s failed", n * sizeof(T), what);
+    const size_t n = std::max<size_t>(need, 1);
+    if (fixed_memory)
+        return fail(CMC_ENOMEM, "%zu bytes for %s are not allocated during a stream capture", n * size, what);
+    void* fresh = nullptr;
+    bool ok = memory.alloc(&fresh, n * size) == cudaSuccess;
+    size_t left = 0;
+    if (!ok && ptr && memory.available(&left) == cudaSuccess && left + cap * size >= n * size) {
+        memory.release(ptr);  // waits for the work that uses it
+        ptr = nullptr;
+        cap = 0;
+        forget_graphs();
+        ok = memory.alloc(&fresh, n * size) == cudaSuccess;
     }
+    if (!ok) {
+        cudaGetLastError();
+        return fail(CMC_ENOMEM, "cudaMalloc of %zu bytes for %s failed", n * size, what);
+    }
+    if (ptr) {
+        memory.release(ptr);
+        forget_graphs();
+    }
+    ptr = fresh;
     cap = n;
     return CMC_OK;
+}
+
+// Captured graphs name the buffers they were captured with.
+void Ctx::forget_graphs() {
+    for (GraphEntry& g : graphs)
+        if (g.exec) cudaGraphExecDestroy(g.exec);
+    graphs.clear();
+}
+
+template <typename T>
+int Ctx::grow(T*& ptr, size_t& cap, size_t need, const char* what) {
+    void* p = ptr;
+    const int rc = grow_bytes(p, cap, need, sizeof(T), what);
+    ptr = static_cast<T*>(p);
+    return rc;
+}
+
+void Ctx::look_for_capture(cudaStream_t st) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &status) != cudaSuccess) cudaGetLastError();
+    fixed_memory = status != cudaStreamCaptureStatusNone;
 }
 
 // Map method of a parameter set.  Direct passes cost 8 AES blocks per Feistel
@@ -1044,7 +1082,7 @@ Ctx::~Ctx() {
     cudaFree(d_ghdr);
     cudaFree(d_job_failed);
     cudaFree(d_key);
-    for (GraphEntry& g : graphs) cudaGraphExecDestroy(g.exec);
+    forget_graphs();
     cudaFreeHost(h_failed);
     cudaFreeHost(h_result);
     cudaFreeHost(h_job);
@@ -1071,6 +1109,7 @@ int Ctx::launch_host(const cmc_params& p, const uint32_t key[44], uint32_t first
     int rc = cuda(cudaSetDevice(device), "cudaSetDevice");
     if (rc) return rc;
     cudaStream_t st = user_stream ? user_stream : stream;
+    look_for_capture(st);
     std::vector<Job> jobs(1);
     if ((rc = make_job(p, first, count, 0, jobs[0]))) return rc;
     std::memcpy(jobs[0].batch_rk, key, 44 * 4);
@@ -1104,6 +1143,7 @@ int Ctx::launch_device(const cmc_params& p, const uint32_t* d_key_in, uint32_t f
     int rc = cuda(cudaSetDevice(device), "cudaSetDevice");
     if (rc) return rc;
     if (count == 0) return cuda(cudaMemsetAsync(d_nfailed, 0, 4, st), "memset count");
+    look_for_capture(st);
     std::vector<Job> jobs(1);
     if ((rc = make_job(p, first, count, 0, jobs[0]))) return rc;
     if ((rc = upload_jobs(jobs, st))) return rc;
@@ -1267,6 +1307,7 @@ int Ctx::run_jobs(const cmc_job* in, uint32_t n, uint64_t* out_failed, uint32_t*
     uint64_t total = 0;
     if ((rc = prepare_jobs(in, n, 0, jobs, order, total, bounds))) return rc;
     cudaStream_t st = user_stream ? user_stream : stream;
+    look_for_capture(st);
     if ((rc = upload_jobs(jobs, st))) return rc;
     if ((rc = grow(d_job_failed, job_failed_cap, n, "job counters"))) return rc;
     const uint64_t dev_cap = out_offsets ? std::min<uint64_t>(cap, total) : 0;
@@ -1311,11 +1352,11 @@ int Ctx::run_jobs(const cmc_job* in, uint32_t n, uint64_t* out_failed, uint32_t*
             graph_state = "replayed";
         } else if (std::find(graph_seen.begin(), graph_seen.end(), key) != graph_seen.end()) {
             cudaGraph_t g = nullptr;
-            capturing = true;
+            capturing = fixed_memory = true;
             rc = cuda(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "begin capture");
             if (!rc) rc = enqueue();
             const cudaError_t e = cudaStreamEndCapture(st, &g);
-            capturing = false;
+            capturing = fixed_memory = false;
             cudaGraphExec_t ex = nullptr;
             const cudaError_t ie = (!rc && e == cudaSuccess && g) ? cudaGraphInstantiate(&ex, g, 0)
                                                                   : cudaErrorUnknown;
@@ -1395,6 +1436,7 @@ int Ctx::autotune(const cmc_job* in, uint32_t n, uint32_t sample_div) {
     uint64_t total = 0;
     if ((rc = prepare_jobs(in, n, sample_div ? sample_div : 64, jobs, order, total, bounds))) return rc;
     cudaStream_t st = user_stream ? user_stream : stream;
+    look_for_capture(st);
     bool any_cached = false;  // does the automatic choice use a round cache anywhere?
     for (const Job& j : jobs) any_cached = any_cached || j.method != kMethodDirect;
     std::vector<TunedPlan> cands{TunedPlan{0, -1, -1}};  // each class under its automatic plan

@@ -70,6 +70,16 @@ const void* wave_kernel(int variant, bool global_cache);
 // Estimated cost of one trial in AES-block equivalents (seeds, map, 0.1 t for the walk).
 double job_cost(const Job& j);
 
+// The device-memory calls of a context's buffers (a test puts its own here).
+struct DeviceMemory {
+    cudaError_t (*alloc)(void**, size_t) = [](void** p, size_t n) { return cudaMalloc(p, n); };
+    cudaError_t (*release)(void*) = [](void* p) { return cudaFree(p); };
+    cudaError_t (*available)(size_t*) = [](size_t* n) {
+        size_t all = 0;
+        return cudaMemGetInfo(n, &all);
+    };
+};
+
 // Planner options chosen by the autotuner for one mix of parameter sets.
 struct TunedPlan {
     uint32_t wg = 0;
@@ -126,6 +136,8 @@ struct Ctx {
     int use_graphs = 1;
     int use_fused = 1;  // batched calls: all plan classes in one persistent launch
     bool capturing = false;
+    DeviceMemory memory;
+    bool fixed_memory = false;  // a stream capture is under way: no buffer is allocated or freed
     std::vector<GraphEntry> graphs;  // most recent last, at most 8
     std::vector<std::string> graph_seen;
     unsigned long long* h_failed = nullptr;  // pinned per-job counts of the last batched call
@@ -147,6 +159,9 @@ struct Ctx {
     int init(int dev);
     int fail(int code, const char* fmt, ...);
     int cuda(cudaError_t e, const char* what);
+    int grow_bytes(void*& ptr, size_t& cap, size_t need, size_t size, const char* what);
+    void forget_graphs();
+    void look_for_capture(cudaStream_t st);
     template <typename T>
     int grow(T*& ptr, size_t& cap, size_t need, const char* what);
     int make_job(const cmc_params& p, uint32_t first, uint32_t count, uint64_t base, Job& j);
