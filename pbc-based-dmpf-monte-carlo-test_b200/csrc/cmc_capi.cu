@@ -1182,23 +1182,33 @@ std::string Ctx::mix_key(const cmc_job* in, uint32_t n) const {
 }
 
 // Everything a captured batched call bakes in: job shapes and counts in table
-// order, plan classes, planner options and the device buffers it touches.
+// order, plan classes, planner options, the buffers it touches and the sizes of
+// those that a replay does not grow first.
 std::string Ctx::graph_key(const std::vector<Job>& jobs, const std::vector<uint32_t>& bounds,
                            uint64_t total, uint64_t dev_cap) const {
     std::string key;
-    char b[160];
-    for (const Job& j : jobs) {
-        snprintf(b, sizeof b, "%u/%u/%u/%u/%u/%u/%u/%u/%llu/%u;", j.mode, j.input_mode, j.pnum, j.k,
-                 j.buckets, j.kick, j.half_bits, j.method, (unsigned long long)j.domain, j.count);
-        key += b;
-    }
-    for (uint32_t x : bounds) key += std::to_string(x) + ",";
-    snprintf(b, sizeof b, "|%llu|%llu|%u/%u/%u/%u/%u/%d/%d/%d/%u/%u/%d|%p/%p/%p/%p/%p/%p/%p",
-             (unsigned long long)total, (unsigned long long)dev_cap, force_wg, force_ng,
-             force_global_slots, force_walkers, max_slots_per_group, force_walker_ctas, force_isolate,
-             force_method, spin_limit, map_chains * 16 + fill_blocks, use_fused + 2 * force_lanes + 128 * force_pool + 1024 * force_waves, (void*)d_jobs, (void*)d_bits, (void*)d_out, (void*)d_slots,
-             (void*)d_ctrl, (void*)d_job_failed, (void*)h_failed);
-    return key + b;
+    auto add = [&](uint64_t v) {
+        key += std::to_string(v);
+        key += '/';
+    };
+    for (const Job& j : jobs)
+        for (uint64_t v : {uint64_t(j.mode), uint64_t(j.input_mode), uint64_t(j.pnum), uint64_t(j.k), uint64_t(j.buckets),
+                           uint64_t(j.kick), uint64_t(j.half_bits), uint64_t(j.method), j.domain, uint64_t(j.count)})
+            add(v);
+    key += '|';
+    for (uint32_t x : bounds) add(x);
+    key += '|';
+    for (int64_t v : {int64_t(total), int64_t(dev_cap), int64_t(force_wg), int64_t(force_ng), int64_t(force_global_slots),
+                      int64_t(force_walkers), int64_t(max_slots_per_group), int64_t(force_walker_ctas),
+                      int64_t(force_isolate), int64_t(force_method), int64_t(spin_limit), int64_t(map_chains),
+                      int64_t(fill_blocks), int64_t(use_fused), int64_t(force_lanes), int64_t(force_waves),
+                      int64_t(force_pool)})
+        add(uint64_t(v));
+    for (const void* p : {(const void*)d_jobs, (const void*)d_bits, (const void*)d_out, (const void*)d_slots,
+                          (const void*)d_job_failed, (const void*)h_failed})
+        add(uint64_t(reinterpret_cast<uintptr_t>(p)));
+    for (size_t n : {bits_cap, slots_cap}) add(n);
+    return key;
 }
 
 int Ctx::prepare_jobs(const cmc_job* in, uint32_t n, uint32_t sample_div, std::vector<Job>& out,

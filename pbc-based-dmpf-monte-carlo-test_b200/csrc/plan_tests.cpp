@@ -113,6 +113,17 @@ void check_graphs() {
     require(!replays() || (reinterpret_cast<uintptr_t>(c.d_slots) == large && c.slots_cap >= 800),
             "a graph replays in its own pool, also after a fallback");
     require(grow_pool(c, 900) == CMC_OK && c.graphs.empty(), "graphs go with the buffer they name");
+
+    // every pointer counts in full
+    for (void** at : {(void**)&c.d_jobs, (void**)&c.d_bits, (void**)&c.d_out, (void**)&c.d_slots,
+                      (void**)&c.d_job_failed, (void**)&c.h_failed}) {
+        void* const was = *at;
+        *at = reinterpret_cast<void*>(0x7ffffffffff0);
+        const std::string a = c.graph_key(jobs, bounds, 0xfffffffe, 0xfffffffe);
+        *at = reinterpret_cast<void*>(0x7ffffffffff1);
+        require(a != c.graph_key(jobs, bounds, 0xfffffffe, 0xfffffffe), "a pointer is part of the key");
+        *at = was;
+    }
 }
 
 }  // namespace
