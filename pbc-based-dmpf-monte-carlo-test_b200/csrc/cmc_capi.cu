@@ -675,10 +675,72 @@ void Ctx::choose_engine(const std::vector<Job>& jobs, const Plan& group, LanePla
     if (waves.ng) lanes = LanePlan{};
 }
 
-// Queue the engine launches over `jobs` (already on the device in d_jobs) --
-// one per plan class, class c covering the job-table range
-// [bounds[c], bounds[c + 1]) and so a contiguous range of global trial
-// indices -- and the compaction of the shared failure bitmap.
+// Plans of a call, one per plan class: class c covers the job-table range
+// [bounds[c], bounds[c + 1]) and so a contiguous range of global trial indices.
+// Several classes of the group engine run as ONE persistent kernel per entry
+// width and walk-slot placement that two or more of them share (both are
+// template parameters), in the order of each kind's heaviest class, unless
+// "fused" is off or a class uses the split engine.  Pooled direct passes, lanes
+// and waves have kernels of their own, as a class alone in its kind.
+//
+// The kernels of a call run one after another in one stream and take the pool in
+// turn; only classes side by side in a fused kernel have regions of their own
+// (64 sets of t = 16..4096 with 65,536 trials each: 2.6 GB, 6.6 with a region
+// for every class).
+int Ctx::plan_launch(const std::vector<Job>& jobs, const std::vector<uint32_t>& bounds, LaunchPlan& lp) {
+    lp = LaunchPlan{};
+    const uint32_t nclass = uint32_t(bounds.size()) - 1;
+    if (nclass < 1 || nclass > kMaxClasses) return fail(CMC_EINVAL, "bad plan classes");
+    lp.plans.resize(nclass);
+    lp.lanes.resize(nclass);
+    lp.waves.resize(nclass);
+    lp.work.assign(nclass, 0.0);
+    lp.trials.assign(nclass, 0.0);
+    lp.region.assign(nclass, 0);
+    bool any_split = false;
+    for (uint32_t c = 0; c < nclass; ++c) {
+        std::vector<Job> part(jobs.begin() + bounds[c], jobs.begin() + bounds[c + 1]);
+        const int rc = plan(part, lp.plans[c]);
+        if (rc) return rc;
+        any_split = any_split || lp.plans[c].walker_ctas;
+        for (const Job& j : part) {
+            lp.trials[c] += double(j.count);
+            lp.work[c] += job_cost(j) * j.count;
+        }
+        if (lp.trials[c] > lp.trials[lp.heaviest]) lp.heaviest = c;
+        choose_engine(part, lp.plans[c], lp.lanes[c], lp.waves[c]);
+        lp.text += (c ? " | " : "") + plan_text + lanes_text(lp.lanes[c]) + waves_text(lp.waves[c]);
+    }
+    const bool fuse = use_fused && nclass > 1 && nclass <= kMaxFusedClasses && !any_split;
+    if (fuse) lp.text = "fused(" + std::to_string(nclass) + ") " + lp.text;
+    std::vector<bool> placed(nclass, false);
+    for (uint32_t lead = 0; lead < nclass && fuse; ++lead) {
+        auto alone = [&](uint32_t c) { return placed[c] || lp.plans[c].pool_stage || lp.lanes[c].warps || lp.waves[c].ng; };
+        if (alone(lead)) continue;
+        std::vector<uint32_t> members;
+        for (uint32_t c = lead; c < nclass; ++c)
+            if (!alone(c) && lp.plans[c].variant == lp.plans[lead].variant &&
+                lp.plans[c].slots_smem == lp.plans[lead].slots_smem)
+                members.push_back(c);
+        if (members.size() < 2) continue;
+        for (uint32_t c : members) placed[c] = true;
+        lp.kernels.push_back(members);
+    }
+    for (uint32_t c = 0; c < nclass; ++c)
+        if (!placed[c]) lp.kernels.push_back({c});
+    for (const std::vector<uint32_t>& members : lp.kernels) {
+        uint64_t at = 0;
+        for (uint32_t c : members) {
+            lp.region[c] = at;
+            at += lp.pool_bytes(c);
+        }
+        lp.pool = std::max(lp.pool, at);
+    }
+    return CMC_OK;
+}
+
+// Queue the engine kernels of a call over `jobs` (already on the device in
+// d_jobs) and the compaction of their shared failure bitmap.
 int Ctx::run(const std::vector<Job>& jobs, uint64_t total, cudaStream_t st, uint32_t value_base,
              uint32_t* d_out, uint32_t* d_count, uint64_t out_cap_now,
              unsigned long long* job_failed, unsigned long long* job_done,
@@ -686,61 +748,18 @@ int Ctx::run(const std::vector<Job>& jobs, uint64_t total, cudaStream_t st, uint
     // launch checks below read cudaGetLastError: start from a clean slate (an
     // earlier non-fatal error, e.g. of a timing query, is not this launch's)
     cudaGetLastError();
-    std::vector<uint32_t> bounds = bounds_in ? *bounds_in : std::vector<uint32_t>{0, uint32_t(jobs.size())};
+    const std::vector<uint32_t> bounds = bounds_in ? *bounds_in : std::vector<uint32_t>{0, uint32_t(jobs.size())};
     const uint32_t nclass = uint32_t(bounds.size()) - 1;
-    if (nclass < 1 || nclass > kMaxClasses) return fail(CMC_EINVAL, "bad plan classes");
-    std::vector<Plan> plans(nclass);
-    std::vector<LanePlan> lanes(nclass);
-    std::vector<WavePlan> waves(nclass);
-    std::vector<double> class_work(nclass, 0.0), class_trials(nclass, 0.0);
-    uint32_t heaviest = 0;
-    uint64_t heaviest_trials = 0;
-    bool any_split = false;
-    std::string text;
-    for (uint32_t c = 0; c < nclass; ++c) {
-        std::vector<Job> part(jobs.begin() + bounds[c], jobs.begin() + bounds[c + 1]);
-        int rc = plan(part, plans[c]);
-        if (rc) return rc;
-        any_split = any_split || plans[c].walker_ctas;
-        uint64_t trials = 0;
-        for (const Job& j : part) {
-            trials += j.count;
-            class_work[c] += job_cost(j) * j.count;
-        }
-        class_trials[c] = double(trials);
-        if (trials > heaviest_trials) {
-            heaviest_trials = trials;
-            heaviest = c;
-        }
-        choose_engine(part, plans[c], lanes[c], waves[c]);
-        text += (c ? " | " : "") + plan_text + lanes_text(lanes[c]) + waves_text(waves[c]);
-    }
-    // Several classes run as ONE persistent launch unless disabled or a class
-    // uses the split engine; the classes then run side by side, so each gets
-    // its own region of the global pool.  Launches one after another reuse one
-    // region in stream order.
-    const bool fuse = use_fused && nclass > 1 && nclass <= kMaxFusedClasses && !any_split;
-    std::vector<uint64_t> region(nclass, 0);
-    uint64_t pool = 0;
-    for (uint32_t c = 0; c < nclass; ++c) {
-        const uint64_t need = waves[c].ng ? waves[c].regions_bytes + waves[c].stock_bytes + waves[c].gcache_bytes
-                              : lanes[c].warps
-                                  ? lanes[c].regions_bytes + lanes[c].stock_bytes
-                                  : (plans[c].gslot_bytes + 255) / 256 * 256 + (plans[c].gcache_bytes + 255) / 256 * 256;
-        if (fuse) {
-            region[c] = pool;
-            pool += need;
-        } else {
-            pool = std::max(pool, need);
-        }
-    }
-    plan_text = fuse ? "fused(" + std::to_string(nclass) + ") " + text : text;
-    const size_t words = (total + 31) / 32;
-    int rc = bitmap(words);
+    LaunchPlan lp;
+    int rc = plan_launch(jobs, bounds, lp);
     if (rc) return rc;
+    const std::vector<Plan>& plans = lp.plans;
+    plan_text = lp.text;
+    const size_t words = (total + 31) / 32;
+    if ((rc = bitmap(words))) return rc;
     uint32_t* const bits = d_bits + kCtrlWords;
     // walk slots, then the groups' round caches, per pool region
-    if (pool && (rc = grow(d_slots, slots_cap, size_t(pool), "slot and cache pool"))) {
+    if (lp.pool && (rc = grow(d_slots, slots_cap, size_t(lp.pool), "slot and cache pool"))) {
         if (rc != CMC_ENOMEM || (force_lanes == 0 && force_waves == 0)) return rc;
         // no room for the tables of the lane or wave engine: the group engine needs less
         const int kept[2] = {force_lanes, force_waves};
@@ -758,7 +777,7 @@ int Ctx::run(const std::vector<Job>& jobs, uint64_t total, cudaStream_t st, uint
     kernels = 0;
     auto class_args = [&](uint32_t c) {
         const Plan& pl = plans[c];
-        char* base = d_slots + region[c];
+        char* base = d_slots + lp.region[c];
         const size_t cache_off = size_t((pl.gslot_bytes + 255) / 256 * 256);
         EngineArgs a{};
         a.jobs = d_jobs;
@@ -796,45 +815,34 @@ int Ctx::run(const std::vector<Job>& jobs, uint64_t total, cudaStream_t st, uint
         a.pool_fold = pl.pool_fold;
         return a;
     };
-    // Fused: one launch per entry width that two or more classes share (the
-    // width is a template parameter of the engine), in the order of each
-    // width's heaviest class; a class alone in its width runs by itself.
-    std::vector<bool> launched(nclass, false);
-    // Classes with pooled direct passes run their own kernel, unfused.
-    for (uint32_t lead = 0; lead < nclass && fuse; ++lead) {
-        if (launched[lead] || plans[lead].pool_stage || lanes[lead].warps || waves[lead].ng) continue;
-        std::vector<uint32_t> members;
-        for (uint32_t c = lead; c < nclass; ++c)
-            if (!launched[c] && !plans[c].pool_stage && !lanes[c].warps && !waves[c].ng && plans[c].variant == plans[lead].variant &&
-                plans[c].slots_smem == plans[lead].slots_smem)
-                members.push_back(c);
-        if (members.size() < 2) continue;
-        FusedArgs fa{};
-        fa.nclass = uint32_t(members.size());
-        uint32_t smem = 0;
-        double all = 0, cum = 0;
-        for (uint32_t c : members) all += class_work[c];
-        for (uint32_t i = 0; i < members.size(); ++i) {
-            const uint32_t c = members[i];
-            launched[c] = true;
-            fa.cls[i] = class_args(c);
-            fa.cost[i] = float(class_work[c] / std::max(1.0, class_trials[c]));
-            fa.first_cta[i] = uint16_t(std::lround(double(sms) * cum / std::max(all, 1e-30)));
-            cum += class_work[c];
-            smem = std::max(smem, plans[c].smem_bytes);
+    for (const std::vector<uint32_t>& members : lp.kernels) {
+        if (members.size() > 1) {
+            FusedArgs fa{};
+            fa.nclass = uint32_t(members.size());
+            uint32_t smem = 0;
+            double all = 0, cum = 0;
+            for (uint32_t c : members) all += lp.work[c];
+            for (uint32_t i = 0; i < members.size(); ++i) {
+                const uint32_t c = members[i];
+                fa.cls[i] = class_args(c);
+                fa.cost[i] = float(lp.work[c] / std::max(1.0, lp.trials[c]));
+                fa.first_cta[i] = uint16_t(std::lround(double(sms) * cum / std::max(all, 1e-30)));
+                cum += lp.work[c];
+                smem = std::max(smem, plans[c].smem_bytes);
+            }
+            fa.first_cta[members.size()] = uint16_t(sms);
+            const Plan& lead = plans[members[0]];
+            const void* fn = fused_engine_kernel(lead.variant, lead.slots_smem);
+            void* args[] = {&fa};
+            if ((rc = cuda(cudaLaunchKernel(fn, dim3(sms), dim3(512), args, smem, st), "fused engine launch")))
+                return rc;
+            ++kernels;
+            continue;
         }
-        fa.first_cta[members.size()] = uint16_t(sms);
-        const void* fn = fused_engine_kernel(plans[lead].variant, plans[lead].slots_smem);
-        void* args[] = {&fa};
-        if ((rc = cuda(cudaLaunchKernel(fn, dim3(sms), dim3(512), args, smem, st), "fused engine launch")))
-            return rc;
-        ++kernels;
-    }
-    for (uint32_t c = 0; c < nclass; ++c) {
-        if (launched[c]) continue;
+        const uint32_t c = members[0];
         const Plan& pl = plans[c];
-        if (waves[c].ng) {
-            const WavePlan& wp = waves[c];
+        if (lp.waves[c].ng) {
+            const WavePlan& wp = lp.waves[c];
             const EngineArgs e = class_args(c);
             WaveArgs a{};
             a.jobs = e.jobs;
@@ -845,7 +853,7 @@ int Ctx::run(const std::vector<Job>& jobs, uint64_t total, cudaStream_t st, uint
             a.fail_bits = e.fail_bits;
             a.job_failed = e.job_failed;
             a.t0 = e.t0;
-            a.regions = d_slots + region[c];
+            a.regions = d_slots + lp.region[c];
             a.region_bytes = wp.region_bytes;
             a.map_off = wp.map_off;
             a.wave = wp.wave;
@@ -866,8 +874,8 @@ int Ctx::run(const std::vector<Job>& jobs, uint64_t total, cudaStream_t st, uint
             ++kernels;
             continue;
         }
-        if (lanes[c].warps) {
-            const LanePlan& lp = lanes[c];
+        if (lp.lanes[c].warps) {
+            const LanePlan& ln = lp.lanes[c];
             const EngineArgs e = class_args(c);
             LaneArgs a{};
             a.jobs = e.jobs;
@@ -878,14 +886,14 @@ int Ctx::run(const std::vector<Job>& jobs, uint64_t total, cudaStream_t st, uint
             a.fail_bits = e.fail_bits;
             a.job_failed = e.job_failed;
             a.t0 = e.t0;
-            a.regions = d_slots + region[c];
-            a.region_bytes = lp.region_bytes;
+            a.regions = d_slots + lp.region[c];
+            a.region_bytes = ln.region_bytes;
             a.hops = kLaneHops;
-            a.stock = reinterpret_cast<uint32_t*>(a.regions + lp.regions_bytes);
-            a.share = lp.share;
+            a.stock = reinterpret_cast<uint32_t*>(a.regions + ln.regions_bytes);
+            a.share = ln.share;
             void* args[] = {&a};
-            if ((rc = cuda(cudaLaunchKernel(lane_kernel(lp.variant), dim3(lp.ctas), dim3(lp.warps * 32), args,
-                                            lp.smem_bytes, st),
+            if ((rc = cuda(cudaLaunchKernel(lane_kernel(ln.variant), dim3(ln.ctas), dim3(ln.warps * 32), args,
+                                            ln.smem_bytes, st),
                            "lane engine launch")))
                 return rc;
             ++kernels;
@@ -921,7 +929,7 @@ int Ctx::run(const std::vector<Job>& jobs, uint64_t total, cudaStream_t st, uint
         if ((rc = cuda(cudaGetLastError(), "compaction launch"))) return rc;
         ++kernels;
     }
-    last_plan = plans[heaviest];
+    last_plan = plans[lp.heaviest];
     ctrl_count = nclass;
     return CMC_OK;
 }

@@ -58,6 +58,27 @@ struct WavePlan {
     double cycles = 0;          // estimated
 };
 
+// How a call runs: its plan classes, the kernels they run in (more than one
+// class: a fused kernel) and their places in the context's pool.
+struct LaunchPlan {
+    std::vector<Plan> plans;
+    std::vector<LanePlan> lanes;
+    std::vector<WavePlan> waves;
+    std::vector<double> work, trials;  // per class: AES blocks, trials
+    std::vector<std::vector<uint32_t>> kernels;
+    std::vector<uint64_t> region;
+    uint64_t pool = 0;
+    uint32_t heaviest = 0;
+    std::string text;
+
+    uint64_t pool_bytes(uint32_t c) const {
+        const auto whole = [](uint64_t n) { return (n + 255) / 256 * 256; };
+        if (waves[c].ng) return whole(waves[c].regions_bytes) + waves[c].stock_bytes + whole(waves[c].gcache_bytes);
+        if (lanes[c].warps) return whole(lanes[c].regions_bytes) + lanes[c].stock_bytes;
+        return whole(plans[c].gslot_bytes) + whole(plans[c].gcache_bytes);
+    }
+};
+
 uint32_t choose_method(uint32_t h, uint64_t domain, double candidates, int force, bool may_allocate);
 // Raises the engine kernels' dynamic shared-memory limit to the device's opt-in maximum.
 int engine_smem_cap(size_t optin);
@@ -169,6 +190,7 @@ struct Ctx {
     LanePlan plan_lanes(const std::vector<Job>& jobs, const Plan& group) const;
     WavePlan plan_waves(const std::vector<Job>& jobs, const Plan& group) const;
     void choose_engine(const std::vector<Job>& jobs, const Plan& group, LanePlan& lanes, WavePlan& waves) const;
+    int plan_launch(const std::vector<Job>& jobs, const std::vector<uint32_t>& bounds, LaunchPlan& lp);
     int upload_jobs(const std::vector<Job>& jobs, cudaStream_t st);
     int run(const std::vector<Job>& jobs, uint64_t total, cudaStream_t st, uint32_t value_base,
             uint32_t* d_out, uint32_t* d_count, uint64_t out_cap, unsigned long long* job_failed,

@@ -126,10 +126,59 @@ void check_graphs() {
     }
 }
 
+cmc_params params(uint32_t mode, uint32_t t, uint32_t ell, uint32_t k, uint32_t buckets, uint32_t kick) {
+    cmc_params p;
+    require(cmc_derive_params(mode, t, ell, k, buckets, kick, CMC_INPUT_AFFINE, &p) == CMC_OK, "parameters");
+    return p;
+}
+
+// The kernels of a call run one after another: they take the pool in turn, and
+// only classes side by side in one kernel have regions of their own.
+void check_regions() {
+    Ctx c;
+    use_fake(c, 0);
+    std::vector<cmc_job> in;
+    for (uint32_t t : {64u, 200u, 300u, 700u, 1024u, 1500u, 2500u, 4000u, 8000u})
+        for (uint32_t k : {2u, 3u, 4u})
+            for (uint32_t count : {40u, 65536u})
+                in.push_back({params(CMC_MODE_BGH25, t, 24, k, t + t / 2, 500), 1, 0, 0, count});
+    uint32_t engines = 0, fused = 0;
+    for (int use_fused : {1, 0}) {
+        c.use_fused = use_fused;
+        std::vector<Job> jobs;
+        std::vector<uint32_t> order, bounds;
+        uint64_t total = 0;
+        LaunchPlan lp;
+        require(c.prepare_jobs(in.data(), uint32_t(in.size()), 0, jobs, order, total, bounds) == CMC_OK &&
+                    c.plan_launch(jobs, bounds, lp) == CMC_OK,
+                "a mix");
+        std::vector<uint32_t> runs(lp.plans.size(), 0);
+        uint64_t largest = 0;
+        for (const auto& members : lp.kernels) {
+            uint64_t sum = 0;
+            for (uint32_t m : members) {
+                ++runs[m];
+                const bool own = lp.lanes[m].warps || lp.waves[m].ng;
+                engines += own;
+                require(!own || members.size() == 1, "lanes and waves have kernels of their own");
+                require(lp.region[m] == sum, "regions of one kernel lie side by side");
+                sum += lp.pool_bytes(m);
+                require(!own || lp.pool_bytes(m) <= c.memory_bytes / 8 + 1024, "an eighth of the device");
+            }
+            fused += members.size() > 1;
+            largest = std::max(largest, sum);
+        }
+        for (uint32_t n : runs) require(n == 1, "every class runs once");
+        require(lp.pool == largest, "the pool holds the largest kernel's regions, not all of them");
+    }
+    require(engines >= 4 && fused >= 1, "the mix has lanes or waves and a fused kernel");
+}
+
 }  // namespace
 
 int main() {
-    const std::pair<const char*, void (*)()> tests[] = {{"buffers", check_grow}, {"graphs", check_graphs}};
+    const std::pair<const char*, void (*)()> tests[] = {{"buffers", check_grow}, {"graphs", check_graphs},
+                                                        {"regions", check_regions}};
     int bad = 0;
     for (auto& [name, test] : tests) {
         try {
