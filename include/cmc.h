@@ -69,7 +69,14 @@ void cmc_host_aes128(const uint32_t rk[44], const uint32_t in[4], uint32_t out[4
 typedef struct cmc_ctx cmc_ctx;
 
 /* Per-device set-up: table upload and the FIPS-197 known-answer test on the
- * device (cuckoo_bench.cu:1090-1095, 332-354).  One context per host thread. */
+ * device (cuckoo_bench.cu:1090-1095, 332-354).  One context per host thread.
+ * A context keeps the device memory of its largest call until cmc_destroy: the
+ * failure bitmap and list, and the tables of the walks, up to an eighth of the
+ * device in the lane and wave engines (13 GB at t = 16384, 65,536 trials).  The
+ * option "pool_bytes" bounds the tables and gives back what is above it.  A call
+ * whose tables do not fit runs in the group engine with fewer walk slots; only
+ * one that fits in no form fails (CMC_ENOMEM).  On a stream that is being
+ * captured nothing is allocated: run the call, or a larger one, before. */
 int cmc_init(int device, cmc_ctx** out);
 int cmc_destroy(cmc_ctx* ctx);
 const char* cmc_last_error(const cmc_ctx* ctx);
@@ -217,7 +224,9 @@ int cmc_server_destroy(cmc_server* server);
  * always, with that many warps per SM), "waves" (-1, the default: likewise the
  * wave engine, whose groups build maps and then walk one trial per thread; 0:
  * never; 1, 2, 4 or 8: with that many groups per SM, fewer where shared memory
- * holds fewer, for PRP half widths up to 16), "pool" (-1, the default:
+ * holds fewer, for PRP half widths up to 16), "pool_bytes" (0, the default:
+ * no limit; else the device memory that this context's tables, walk slots and
+ * round caches may take, servers apart), "pool" (-1, the default:
  * one-warp groups whose jobs all take direct passes with 16-bit Feistel
  * halves and shared-memory walk slots keep three trials in flight and stage
  * their maps; 0: one trial at a time; 1 as -1 -- such plans run in a kernel

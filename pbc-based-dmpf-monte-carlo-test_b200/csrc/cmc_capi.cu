@@ -408,15 +408,22 @@ int Ctx::plan(const std::vector<Job>& jobs, Plan& pl) {
         }
     }
     if (!pl.slots_smem) pl.pool_stage = pl.pool_fold = 0;
-    if (!pl.slots_smem && !wide && !pl.walker_ctas) {
-        // global slots of items (item_slots in cmc_engine.cu): [B x 8 bytes]
-        // [t x 8 bytes], as many as the caller's budget
-        // holds beside the round caches
-        pl.bins_bytes = round_up(max_b * 8, 16);
-        pl.slot_stride = round_up(pl.bins_bytes + max_t * 8, 128);
-        const uint64_t caches = any_gcache ? uint64_t(sms) * pl.ng * (16u << max_gcache_h) : 0;
-        const uint64_t fit = (slot_budget - std::min(slot_budget, caches)) / (uint64_t(sms) * pl.slot_stride);
-        if (pl.ns > fit) pl.ns = std::max<uint32_t>(1, uint32_t(fit) / pl.ng) * pl.ng;
+    if (!pl.slots_smem && !pl.walker_ctas) {
+        if (!wide) {
+            // global slots of items (item_slots in cmc_engine.cu): [B x 8 bytes]
+            // [t x 8 bytes]
+            pl.bins_bytes = round_up(max_b * 8, 16);
+            pl.slot_stride = round_up(pl.bins_bytes + max_t * 8, 128);
+        }
+        // as many as the budget holds beside the round caches, down to one per
+        // group and then one group
+        auto fit = [&](uint32_t groups) {
+            const uint64_t caches = any_gcache ? uint64_t(sms) * groups * (16u << max_gcache_h) : 0;
+            return (slot_budget - std::min(slot_budget, caches)) / (uint64_t(sms) * pl.slot_stride);
+        };
+        while (pl.ng > 1 && fit(pl.ng) < pl.ng) --pl.ng;
+        if (pl.ns > fit(pl.ng)) pl.ns = std::max<uint32_t>(1, uint32_t(fit(pl.ng)) / pl.ng) * pl.ng;
+        if (pl.ns % pl.ng) pl.ns -= pl.ns % pl.ng;
     }
     pl.group_off = kEngineTableBytes + kCtaSharedBytes;
     pl.slots_off = pl.group_off + pl.ng * pl.group_bytes;
@@ -649,6 +656,7 @@ WavePlan Ctx::plan_waves(const std::vector<Job>& jobs, const Plan& group) const 
 void Ctx::choose_engine(const std::vector<Job>& jobs, const Plan& group, LanePlan& lanes, WavePlan& waves) const {
     lanes = LanePlan{};
     waves = WavePlan{};
+    if (group_engine) return;
     const bool group_options = force_wg || force_ng || force_global_slots || force_walkers ||
                                force_walker_ctas >= 0 || force_isolate >= 0 || force_method >= 0 ||
                                force_pool >= 0 || max_slots_per_group != 8 || map_chains || fill_blocks;
@@ -739,6 +747,56 @@ int Ctx::plan_launch(const std::vector<Job>& jobs, const std::vector<uint32_t>& 
     return CMC_OK;
 }
 
+// Room for n bytes of tables, walk slots and round caches.  A size that the
+// device did not have is asked for again only when there is more room than there
+// was then, so that a context short of memory does not try on every call.
+int Ctx::reserve_pool(uint64_t n) {
+    if (n == 0 || (n <= slots_cap && d_slots)) return CMC_OK;
+    if (n > pool_limit)
+        return fail(CMC_ENOMEM, "%llu bytes of walk tables exceed the option pool_bytes", (unsigned long long)n);
+    auto room = [&]() {
+        size_t left = 0;
+        return memory.available(&left) == cudaSuccess ? uint64_t(left) + slots_cap : 0;
+    };
+    if (refused && n >= refused && !fixed_memory && room() <= refused_room)
+        return fail(CMC_ENOMEM, "%llu bytes of walk tables do not fit the device", (unsigned long long)n);
+    const int rc = grow(d_slots, slots_cap, size_t(n), "slot and cache pool");
+    if (rc == CMC_ENOMEM && !fixed_memory) {
+        if (!refused || n < refused) refused = n;
+        refused_room = room();
+    } else if (rc == CMC_OK && n >= refused) {
+        refused = 0;
+    }
+    return rc;
+}
+
+// The plan of a call and the pool it needs.  Where the device, or the caller's
+// limit, has no room for it: the group engine alone, and then with half as many
+// walk slots each time (t = 16384, B = 65535, 200 trials: 0.35 GB of waves, else
+// 12.4 GB of walk slots at most and 0.1 at least).
+int Ctx::fit_launch(const std::vector<Job>& jobs, const std::vector<uint32_t>& bounds, LaunchPlan& lp) {
+    int rc = plan_launch(jobs, bounds, lp);
+    if (rc || (rc = reserve_pool(lp.pool)) != CMC_ENOMEM) return rc;
+    const std::string why = err;
+    const uint64_t budget = slot_budget;
+    uint64_t smallest = lp.pool;  // that was refused
+    group_engine = true;
+    for (;;) {
+        if ((rc = plan_launch(jobs, bounds, lp))) break;
+        if (lp.pool < smallest) {
+            if ((rc = reserve_pool(lp.pool)) != CMC_ENOMEM) break;
+            smallest = lp.pool;
+        } else if (slot_budget < (1u << 20)) {
+            rc = fail(CMC_ENOMEM, "%s", why.c_str());
+            break;
+        }
+        slot_budget = std::min(slot_budget, lp.pool) / 2;
+    }
+    group_engine = false;
+    slot_budget = budget;
+    return rc;
+}
+
 // Queue the engine kernels of a call over `jobs` (already on the device in
 // d_jobs) and the compaction of their shared failure bitmap.
 int Ctx::run(const std::vector<Job>& jobs, uint64_t total, cudaStream_t st, uint32_t value_base,
@@ -751,25 +809,13 @@ int Ctx::run(const std::vector<Job>& jobs, uint64_t total, cudaStream_t st, uint
     const std::vector<uint32_t> bounds = bounds_in ? *bounds_in : std::vector<uint32_t>{0, uint32_t(jobs.size())};
     const uint32_t nclass = uint32_t(bounds.size()) - 1;
     LaunchPlan lp;
-    int rc = plan_launch(jobs, bounds, lp);
+    int rc = fit_launch(jobs, bounds, lp);
     if (rc) return rc;
     const std::vector<Plan>& plans = lp.plans;
     plan_text = lp.text;
     const size_t words = (total + 31) / 32;
     if ((rc = bitmap(words))) return rc;
     uint32_t* const bits = d_bits + kCtrlWords;
-    // walk slots, then the groups' round caches, per pool region
-    if (lp.pool && (rc = grow(d_slots, slots_cap, size_t(lp.pool), "slot and cache pool"))) {
-        if (rc != CMC_ENOMEM || (force_lanes == 0 && force_waves == 0)) return rc;
-        // no room for the tables of the lane or wave engine: the group engine needs less
-        const int kept[2] = {force_lanes, force_waves};
-        force_lanes = force_waves = 0;
-        rc = run(jobs, total, st, value_base, d_out, d_count, out_cap_now, job_failed, job_done, bounds_in,
-                 read_back);
-        force_lanes = kept[0];
-        force_waves = kept[1];
-        return rc;
-    }
     if ((rc = cuda(cudaMemsetAsync(d_bits, 0, (kCtrlWords + words) * 4, st), "memset ctrl and bitmap"))) return rc;
     // timing events stay out of captured graphs: a replay records them
     // around the graph launch instead
@@ -1210,7 +1256,7 @@ std::string Ctx::graph_key(const std::vector<Job>& jobs, const std::vector<uint3
                       int64_t(force_walkers), int64_t(max_slots_per_group), int64_t(force_walker_ctas),
                       int64_t(force_isolate), int64_t(force_method), int64_t(spin_limit), int64_t(map_chains),
                       int64_t(fill_blocks), int64_t(use_fused), int64_t(force_lanes), int64_t(force_waves),
-                      int64_t(force_pool)})
+                      int64_t(force_pool), int64_t(pool_limit)})
         add(uint64_t(v));
     for (const void* p : {(const void*)d_jobs, (const void*)d_bits, (const void*)d_out, (const void*)d_slots,
                           (const void*)d_job_failed, (const void*)h_failed})
@@ -1593,6 +1639,16 @@ int cmc_set_option(cmc_ctx* ctx, const char* name, int64_t value) {
     else if (n == "walker_ctas" && value >= -1 && value < c->sms) c->force_walker_ctas = int(value);
     else if (n == "slots_per_group" && value >= 0 && value <= 32)
         c->max_slots_per_group = value ? uint32_t(value) : 8u;
+    else if (n == "pool_bytes" && value >= 0) {
+        c->pool_limit = value ? uint64_t(value) : ~0ull;
+        if (c->slots_cap > c->pool_limit) {
+            cudaSetDevice(c->device);
+            c->memory.release(c->d_slots);  // waits for the work that uses it
+            c->d_slots = nullptr;
+            c->slots_cap = 0;
+            c->forget_graphs();
+        }
+    }
     else if (n == "spin_limit" && value >= 0 && value <= 0xffffffffLL)
         c->spin_limit = value ? uint32_t(value) : (1u << 26);
     else return c->fail(CMC_EINVAL, "unknown option or value out of range: %s=%lld", name, (long long)value);

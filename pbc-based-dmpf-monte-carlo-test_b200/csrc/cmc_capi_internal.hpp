@@ -169,7 +169,10 @@ struct Ctx {
     int force_waves = -1;   // wave engine: -1 auto, 0 off, N groups per CTA
     int force_pool = -1;    // pooled direct passes: -1 auto, 0 off, 1 on where they apply
     bool plan_no_dfold = false;  // plan() re-run without room for direct passes' fold tables
-    uint64_t slot_budget = ~0ull;  // bytes for global walk slots and round caches (a server's budget)
+    uint64_t slot_budget = ~0ull;  // bytes for global walk slots and round caches
+    uint64_t pool_limit = ~0ull;   // bytes the pool may take (option pool_bytes)
+    uint64_t refused = 0, refused_room = 0;  // a pool the device did not have, and the room it had then
+    bool group_engine = false;     // no lanes or waves: the call is short of memory
     bool group_only = false;   // the caller has no lane or wave engine (a server's launches)
     bool may_allocate = true;  // false: no global round cache, global slots only if unavoidable
     uint32_t spin_limit = 1u << 26;
@@ -191,6 +194,8 @@ struct Ctx {
     WavePlan plan_waves(const std::vector<Job>& jobs, const Plan& group) const;
     void choose_engine(const std::vector<Job>& jobs, const Plan& group, LanePlan& lanes, WavePlan& waves) const;
     int plan_launch(const std::vector<Job>& jobs, const std::vector<uint32_t>& bounds, LaunchPlan& lp);
+    int reserve_pool(uint64_t n);
+    int fit_launch(const std::vector<Job>& jobs, const std::vector<uint32_t>& bounds, LaunchPlan& lp);
     int upload_jobs(const std::vector<Job>& jobs, cudaStream_t st);
     int run(const std::vector<Job>& jobs, uint64_t total, cudaStream_t st, uint32_t value_base,
             uint32_t* d_out, uint32_t* d_count, uint64_t out_cap, unsigned long long* job_failed,

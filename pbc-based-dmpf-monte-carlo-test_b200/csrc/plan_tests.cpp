@@ -174,11 +174,72 @@ void check_regions() {
     require(engines >= 4 && fused >= 1, "the mix has lanes or waves and a fused kernel");
 }
 
+// One call of the jobs as Ctx::run plans it; the text of its plan.
+std::string fitted(Ctx& c, const std::vector<cmc_job>& in, LaunchPlan& lp) {
+    std::vector<Job> jobs;
+    std::vector<uint32_t> order, bounds;
+    uint64_t total = 0;
+    require(c.prepare_jobs(in.data(), uint32_t(in.size()), 0, jobs, order, total, bounds) == CMC_OK, "jobs");
+    const int rc = c.fit_launch(jobs, bounds, lp);
+    if (rc) return std::to_string(rc);
+    require(lp.pool <= c.slots_cap, "the pool holds the plan");
+    return lp.text;
+}
+
+// A call whose pool does not fit takes the group engine with fewer walk slots,
+// and an equal call after it allocates nothing.
+void check_short_memory() {
+    const auto has = [](const std::string& text, const char* what) { return text.find(what) != std::string::npos; };
+    const uint64_t gb = 1000000000;
+    // 13 GB of lane tables; the walk slots of a launch of 200 trials
+    const std::vector<cmc_job> lanes{{params(CMC_MODE_BGH25, 16384, 28, 3, 24576, 1000), 4, 0, 0, 65536}};
+    const std::vector<cmc_job> waves{{params(CMC_MODE_BGH25, 16384, 20, 3, 65535, 500), 4, 0, 0, 200}};
+    const std::vector<cmc_job> wide{{params(CMC_MODE_DRRT18, 50000, 20, 3, 70000, 500), 4, 0, 0, 300}};
+    for (const auto* in : {&lanes, &waves, &wide})
+        for (uint64_t size : {180 * gb, 5 * gb, 2 * gb, gb / 2, gb / 4}) {
+            Ctx c;
+            use_fake(c, size);
+            std::string first;
+            for (int call = 0; call < 3; ++call) {
+                LaunchPlan lp;
+                const uint32_t calls = g_device.allocs + g_device.releases;
+                const std::string text = fitted(c, *in, lp);
+                require(has(text, "engine="), "a call that fits in some form succeeds");
+                require(size < 180 * gb || in == &wide || has(text, "->"), "the engine of choice where there is room");
+                require(call == 0 || (text == first && g_device.allocs + g_device.releases == calls),
+                        "an equal call takes the same plan and allocates nothing");
+                require(g_device.live.size() == 1, "one pool");
+                for (const Plan& pl : lp.plans)
+                    require(pl.ng >= 1 && pl.ns >= pl.ng && pl.ns % pl.ng == 0, "slots for every group");
+                first = text;
+            }
+            // under a capture the same plan, without a call
+            c.fixed_memory = true;
+            LaunchPlan lp;
+            require(fitted(c, *in, lp) == first, "the plan of a capture");
+            c.fixed_memory = false;
+            // more room: the engine of choice again
+            g_device.size = 180 * gb;
+            if (in != &wide) require(has(fitted(c, *in, lp), "->"), "memory that was short is not short for good");
+        }
+    // nothing fits
+    Ctx c;
+    use_fake(c, 1000000);
+    LaunchPlan lp;
+    require(fitted(c, lanes, lp) == std::to_string(CMC_ENOMEM) && !c.group_engine && c.slot_budget == ~0ull,
+            "too little memory for any form");
+    // the caller's limit
+    use_fake(c, 180 * gb);
+    c.pool_limit = gb;
+    require(!has(fitted(c, lanes, lp), "->") && lp.pool <= gb, "a plan within the limit");
+}
+
 }  // namespace
 
 int main() {
     const std::pair<const char*, void (*)()> tests[] = {{"buffers", check_grow}, {"graphs", check_graphs},
-                                                        {"regions", check_regions}};
+                                                        {"regions", check_regions},
+                                                        {"short memory", check_short_memory}};
     int bad = 0;
     for (auto& [name, test] : tests) {
         try {
