@@ -141,7 +141,12 @@ int cmc_autotune(cmc_ctx* ctx, const cmc_job* jobs, uint32_t njobs, uint32_t sam
  * journal (when a directory was given; an existing journal there is
  * resumed).  A budget runs as the first ceil(trials / 2^batch_bits) batches
  * of an experiment of 2^ceil(log2 trials) trials, so it is rounded up to
- * whole batches.  A job's failures are the same alone and in the mix. */
+ * whole batches.  A job's failures are the same alone and in the mix.
+ * mem_budget_bytes bounds the device memory of job state, walk slots and round
+ * caches (a resident launch's job ring and failure bits, 4 MB, come on top).  A
+ * job is admitted while twice what its walk slots and caches take at full number
+ * fits beside the other active jobs'; a launch takes fewer slots where that, or
+ * the jobs that walk in shared memory when alone, would exceed the budget. */
 typedef struct cmc_server cmc_server;
 int cmc_server_create(cmc_ctx* ctx, uint32_t max_jobs, uint64_t mem_budget_bytes,
                       uint32_t batch_bits, uint64_t max_iteration_trials, cmc_server** out);

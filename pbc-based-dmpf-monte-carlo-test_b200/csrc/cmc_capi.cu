@@ -277,7 +277,8 @@ int Ctx::plan(const std::vector<Job>& jobs, Plan& pl) {
     const uint32_t budget = uint32_t(smem_optin) - kEngineTableBytes - kCtaSharedBytes;
     uint32_t cap_ng = force_ng;
     // Short launches (longer ones of these shapes run in the lane or wave engine)
-    // and callers that have this engine only: split all 15 warps beside the
+    // and calls without allocation, but not a server's, whose plans must not
+    // depend on the counts: split all 15 warps beside the
     // walker into as many groups as shared memory holds with enough walk slots
     // -- 4 per group up to 28 -- and as there are trials for.  More, smaller
     // groups overlap their serial set-ups and barriers.  Measured on B200
@@ -291,7 +292,7 @@ int Ctx::plan(const std::vector<Job>& jobs, Plan& pl) {
     // N=2^16: 21 slots 1.22 ms, 16 slots 1.40).  64-bit domains, whose set-up is
     // longest, keep their one-warp groups (t=391, k=4: 1.96 against 2.13 ms).
     const double per_sm = work / sms;
-    const bool short_launch = !may_allocate || group_only || per_sm <= 200;
+    const bool short_launch = !served && (!may_allocate || per_sm <= 200);
     if (short_launch && !force_wg && !force_ng && !force_walkers && force_isolate < 0 &&
         !pl.walker_ctas && !any_gcache && !wide_domain) {
         const bool direct_pool = force_pool != 0 && !any_cache;
@@ -371,6 +372,9 @@ int Ctx::plan(const std::vector<Job>& jobs, Plan& pl) {
     avg_cost = work > 0 ? avg_cost / work : 1;
     const double probes = std::max(1.0, 2.4 * avg_probe_work);
     const double produce = (any_gcache ? 0.2 : 0.157) / std::max(1.0, avg_cost);
+    const auto caches = [&](uint32_t groups) {  // round caches of all CTAs
+        return any_gcache ? uint64_t(sms) * groups * (16u << max_gcache_h) : 0;
+    };
     pl.slots_smem = false;
     for (uint32_t g = ng; !pl.walker_ctas && !force_global_slots &&
                           g >= std::max<uint32_t>(1, (ng + 1) / 2); --g) {
@@ -407,6 +411,28 @@ int Ctx::plan(const std::vector<Job>& jobs, Plan& pl) {
             pl.ns = ns_g;
         }
     }
+    // (the split engine has one pool of slots, the others one per CTA)
+    pl.claim_bytes = pl.slots_smem ? 0 : uint64_t(pl.walker_ctas ? 1 : sms) * pl.ns * pl.slot_stride;
+    pl.claim_bytes = (pl.claim_bytes + 255) / 256 * 256 + caches(pl.ng);
+    pl.reduced = false;
+    if (!pl.slots_smem && !pl.walker_ctas && !force_global_slots &&
+        uint64_t(sms) * (wide ? pl.slot_stride : 8ull * (max_b + max_t)) + caches(1) > slot_budget) {
+        // not even one global slot per CTA is within the budget
+        for (uint32_t g = groups_for(1); g >= 1 && !pl.slots_smem; --g) {
+            const uint32_t left = budget - g * pl.group_bytes;
+            const uint32_t s = std::min<uint32_t>({left / pl.slot_stride / g, 32 / g, max_slots_per_group});
+            if (s < 1) continue;
+            pl.slots_smem = true;
+            pl.nw = 1;
+            pl.ng = g;
+            pl.ns = g * s;
+        }
+    }
+    if (pl.slots_smem && caches(pl.ng) > slot_budget) {
+        const uint32_t s = pl.ns / pl.ng;
+        while (pl.ng > 1 && caches(pl.ng) > slot_budget) --pl.ng;
+        pl.ns = pl.ng * s;
+    }
     if (!pl.slots_smem) pl.pool_stage = pl.pool_fold = 0;
     if (!pl.slots_smem && !pl.walker_ctas) {
         if (!wide) {
@@ -418,9 +444,9 @@ int Ctx::plan(const std::vector<Job>& jobs, Plan& pl) {
         // as many as the budget holds beside the round caches, down to one per
         // group and then one group
         auto fit = [&](uint32_t groups) {
-            const uint64_t caches = any_gcache ? uint64_t(sms) * groups * (16u << max_gcache_h) : 0;
-            return (slot_budget - std::min(slot_budget, caches)) / (uint64_t(sms) * pl.slot_stride);
+            return (slot_budget - std::min(slot_budget, caches(groups))) / (uint64_t(sms) * pl.slot_stride);
         };
+        pl.reduced = fit(pl.ng) < pl.ns;
         while (pl.ng > 1 && fit(pl.ng) < pl.ng) --pl.ng;
         if (pl.ns > fit(pl.ng)) pl.ns = std::max<uint32_t>(1, uint32_t(fit(pl.ng)) / pl.ng) * pl.ng;
         if (pl.ns % pl.ng) pl.ns -= pl.ns % pl.ng;
@@ -1205,6 +1231,47 @@ int Ctx::launch_device(const cmc_params& p, const uint32_t* d_key_in, uint32_t f
                    "copy batch key")))
         return rc;
     return run(jobs, count, st, first, d_offsets, d_nfailed, count, nullptr, nullptr);
+}
+
+// Plan of a server's launch over `shapes` within `budget` bytes.  Admission,
+// size classes and launches plan the same jobs with different counts (trials are
+// granted step by step), so a served plan depends on the shapes alone: no split
+// for short launches.  A resident launch walks global slots with four isolated
+// warps, whose number does not depend on the table size, so that jobs that come
+// later fit; where not even one such slot per SM is within the budget it keeps
+// the plan of an iteration, unpooled.
+int Ctx::plan_served(const std::vector<Job>& shapes, uint64_t budget, bool resident, Plan& pl, uint64_t& pool) {
+    const uint64_t was_budget = slot_budget;
+    const uint32_t gs = force_global_slots, wk = force_walkers;
+    const int iso = force_isolate, wc = force_walker_ctas, fp = force_pool;
+    served = true;
+    slot_budget = budget;
+    const auto measured = [&](int rc) {
+        pool = (pl.gslot_bytes + 255) / 256 * 256 + pl.gcache_bytes;
+        return rc;
+    };
+    int rc;
+    if (resident) {
+        force_global_slots = 1;
+        force_isolate = 1;
+        force_walkers = 4;
+        force_walker_ctas = 0;
+        rc = measured(plan(shapes, pl));
+        force_global_slots = gs;
+        force_walkers = wk;
+        force_isolate = iso;
+        if (rc == CMC_OK && pool > budget) {
+            force_pool = 0;
+            rc = measured(plan(shapes, pl));
+            force_pool = fp;
+        }
+        force_walker_ctas = wc;
+    } else {
+        rc = measured(plan(shapes, pl));
+    }
+    served = false;
+    slot_budget = was_budget;
+    return rc;
 }
 
 // Estimated AES-block cost of one trial of a job (map build + seeds), used to

@@ -27,6 +27,10 @@ struct Plan {
     uint32_t slot_stride = 0, bins_bytes = 0, group_bytes = 0;
     uint32_t group_off = 0, slots_off = 0, smem_bytes = 0, threads = 0, ctas = 0;
     int variant = 0;  // 0: u16 map/bins, 1: u32 map/bins, 2: u32 + 64-bit PRP domain
+    // What a server counts for this plan: its walk slots at full number and, for
+    // 16-bit tables, without their items' buckets, and its round caches.
+    uint64_t claim_bytes = 0;
+    bool reduced = false;         // fewer walk slots than planned: Ctx::slot_budget
     uint64_t gslot_bytes = 0;     // global walk slots (0: slots in shared memory)
     uint32_t gcache_stride = 0;   // u16 entries per group's global round cache
     uint64_t gcache_bytes = 0;    // all groups' global round caches
@@ -173,7 +177,7 @@ struct Ctx {
     uint64_t pool_limit = ~0ull;   // bytes the pool may take (option pool_bytes)
     uint64_t refused = 0, refused_room = 0;  // a pool the device did not have, and the room it had then
     bool group_engine = false;     // no lanes or waves: the call is short of memory
-    bool group_only = false;   // the caller has no lane or wave engine (a server's launches)
+    bool served = false;       // planning a server's launch (plan_served)
     bool may_allocate = true;  // false: no global round cache, global slots only if unavoidable
     uint32_t spin_limit = 1u << 26;
     uint32_t map_chains = 0;  // lookup chains per lane from a round cache (0: automatic)
@@ -190,6 +194,7 @@ struct Ctx {
     int grow(T*& ptr, size_t& cap, size_t need, const char* what);
     int make_job(const cmc_params& p, uint32_t first, uint32_t count, uint64_t base, Job& j);
     int plan(const std::vector<Job>& jobs, Plan& pl);
+    int plan_served(const std::vector<Job>& shapes, uint64_t budget, bool resident, Plan& pl, uint64_t& pool);
     LanePlan plan_lanes(const std::vector<Job>& jobs, const Plan& group) const;
     WavePlan plan_waves(const std::vector<Job>& jobs, const Plan& group) const;
     void choose_engine(const std::vector<Job>& jobs, const Plan& group, LanePlan& lanes, WavePlan& waves) const;

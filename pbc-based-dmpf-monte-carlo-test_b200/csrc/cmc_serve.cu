@@ -347,6 +347,10 @@ struct Server {
         return resident ? resident_setup() : CMC_OK;  // the first step then allocates nothing
     }
 
+    // Device memory for the walk slots and round caches of the launches in
+    // flight: one resident launch, or two iterations.
+    uint64_t pool_room() const { return mem_budget - fixed_bytes; }
+
     // Plan for a set of active parameter sets; returns the global pool bytes
     // the plan needs: walk slots (0 for shared-memory slots), then round caches.
     int plan_for(const std::vector<uint32_t>& ids, Plan& pl, std::vector<Job>& shapes, uint64_t& pool,
@@ -358,14 +362,10 @@ struct Server {
             if (rc) return fail(rc, ctx->err);
             shapes.push_back(j);
         }
-        // walk slots give way to the budget, of which an iteration gets half
-        ctx->slot_budget = (mem_budget - fixed_bytes) / (for_resident ? 1 : 2);
-        ctx->slot_budget -= std::min<uint64_t>(ctx->slot_budget, 256);  // the caches' alignment
-        int rc = ctx->plan(shapes, pl);
-        ctx->slot_budget = ~0ull;
-        if (rc) return fail(rc, ctx->err);
-        pool = cache_offset(pl) + pl.gcache_bytes;
-        return CMC_OK;
+        // less the alignment of the caches
+        const uint64_t budget = pool_room() / (for_resident ? 1 : 2);
+        const int rc = ctx->plan_served(shapes, budget - std::min<uint64_t>(budget, 256), for_resident, pl, pool);
+        return rc ? fail(rc, ctx->err) : CMC_OK;
     }
 
     static uint64_t cache_offset(const Plan& pl) { return (pl.gslot_bytes + 255) / 256 * 256; }
@@ -414,7 +414,8 @@ struct Server {
             std::vector<Job> one(1);
             one[0] = probe;
             Plan pl;
-            if ((rc = ctx->plan(one, pl))) return fail(rc, ctx->err);
+            uint64_t pool = 0;
+            if ((rc = ctx->plan_served(one, pool_room() / 2, false, pl, pool))) return fail(rc, ctx->err);
             j.global_slots = pl.slots_smem ? 0 : 1;
             // a trial's walk is ~2.4 t probes of ~300 (shared) or ~3000 (global)
             // cycles; expressed in blocks of GPU throughput (~4e10 blocks/s at 2 GHz)
@@ -475,7 +476,9 @@ struct Server {
             uint64_t pool = 0;
             int rc = plan_for(ids, pl, shapes, pool);
             if (rc) return rc;
-            if (fixed_bytes + 2 * pool > mem_budget) {  // two iterations in flight
+            // two iterations in flight; what runs then keeps within the budget
+            // (plan_served), with fewer slots where the claim is all of it
+            if (fixed_bytes + 2 * pl.claim_bytes > mem_budget) {
                 if (ids.size() == 1)
                     return fail(CMC_ENOMEM, "job " + std::to_string(id) +
                                                 " alone needs more device memory than the budget");
@@ -592,20 +595,34 @@ struct Server {
 
     // Queue one iteration on b's stream: grants -> scheduler -> engine ->
     // compaction -> read-back into pinned memory.
-    int issue(StepBuf& b, const std::vector<Grant>& grants, const std::vector<uint32_t>& grant_jobs) {
+    int issue(StepBuf& b, std::vector<Grant>& grants, std::vector<uint32_t>& grant_jobs) {
         int rc = CMC_OK;
         cudaStream_t st = b.stream;
-        std::vector<uint32_t> weights;  // the plan weighs each shape by its granted trials
-        for (const Grant& g : grants) weights.push_back(g.trials);
         Plan pl;
         std::vector<Job> shapes;
         uint64_t pool = 0;
-        if ((rc = plan_for(grant_jobs, pl, shapes, pool, &weights))) return rc;
+        for (;;) {
+            std::vector<uint32_t> weights;  // the plan weighs each shape by its granted trials
+            for (const Grant& g : grants) weights.push_back(g.trials);
+            if ((rc = plan_for(grant_jobs, pl, shapes, pool, &weights))) return rc;
+            if (pool <= pool_room() / 2) break;
+            // a mix that the budget does not hold in any form: the last grant waits
+            if (grants.size() == 1)
+                return fail(CMC_ENOMEM, "job " + std::to_string(grant_jobs[0]) +
+                                            " alone needs more device memory than the budget");
+            jobs[grant_jobs.back()].next -= grants.back().trials;
+            grants.pop_back();
+            grant_jobs.pop_back();
+        }
+        if (d_rpool && !r_running) {  // of an earlier resident launch
+            cudaFree(d_rpool);
+            d_rpool = nullptr;
+            rpool_bytes = 0;
+        }
         if (pool > b.pool_bytes) {
             // grow with headroom (within the budget): each regrowth's cudaFree
             // waits for the device and drains the pipeline
-            const uint64_t room = mem_budget > fixed_bytes ? (mem_budget - fixed_bytes) / 2 : pool;
-            const uint64_t want = std::max(pool, std::min<uint64_t>(pool + pool / 2, room));
+            const uint64_t want = std::max(pool, std::min<uint64_t>(pool + pool / 2, pool_room() / 2));
             cudaFree(b.d_pool);
             b.d_pool = nullptr;
             b.pool_bytes = 0;
@@ -827,25 +844,18 @@ struct Server {
         return CMC_OK;
     }
 
-    // Plan of a resident launch: global walk slots with four isolated walker
-    // warps (slot count does not depend on the table size), sized for every
-    // active and queued job.
+    // Plan of a resident launch (Ctx::plan_served), sized for every active job
+    // and, where the budget holds all walk slots then, every queued one.
     int resident_plan(Plan& pl, uint64_t& pool) {
         std::vector<uint32_t> ids = active_ids();
-        for (uint32_t id : queue) ids.push_back(id);
-        const uint32_t gs = ctx->force_global_slots, wk = ctx->force_walkers;
-        const int iso = ctx->force_isolate, wc = ctx->force_walker_ctas;
-        ctx->force_global_slots = 1;
-        ctx->force_isolate = 1;
-        ctx->force_walkers = 4;
-        ctx->force_walker_ctas = 0;
         std::vector<Job> shapes;
-        const int rc = plan_for(ids, pl, shapes, pool, nullptr, true);
-        ctx->force_global_slots = gs;
-        ctx->force_walkers = wk;
-        ctx->force_isolate = iso;
-        ctx->force_walker_ctas = wc;
-        return rc;
+        if (!queue.empty()) {
+            for (uint32_t id : queue) ids.push_back(id);
+            const int rc = plan_for(ids, pl, shapes, pool, nullptr, true);
+            if (rc || (!pl.reduced && !pl.slots_smem && pool <= pool_room())) return rc;
+            ids = active_ids();
+        }
+        return plan_for(ids, pl, shapes, pool, nullptr, true);
     }
 
     // Can job `id` run under the running launch's plan (slot size, entry width)?
@@ -857,7 +867,7 @@ struct Server {
         const uint32_t entry = r_plan.variant ? 4 : 2;
         const Job& j = shapes[0];
         // slots of items for 16-bit tables (Ctx::plan), else bins and a k-fold map
-        const bool items = r_plan.variant == 0;
+        const bool items = r_plan.variant == 0 && !r_plan.slots_smem;
         const uint64_t bins = (uint64_t(j.buckets) * (items ? 8 : entry) + 15) / 16 * 16;
         const uint64_t map = items ? uint64_t(j.pnum) * 8 : (uint64_t(j.pnum) * j.k * entry + 15) / 16 * 16;
         // the map of every slot starts at the plan's bins_bytes
@@ -930,6 +940,13 @@ struct Server {
         uint64_t pool = 0;
         int rc = resident_plan(pl, pool);
         if (rc) return rc;
+        if (pool > pool_room()) return fail(CMC_ENOMEM, "the active jobs need more device memory than the budget");
+        for (StepBuf& b : bufs)
+            if (b.d_pool && !b.busy) {  // of earlier iterations
+                cudaFree(b.d_pool);
+                b.d_pool = nullptr;
+                b.pool_bytes = 0;
+            }
         if (pool > rpool_bytes) {
             cudaFree(d_rpool);
             d_rpool = nullptr;

@@ -234,12 +234,92 @@ void check_short_memory() {
     require(!has(fitted(c, lanes, lp), "->") && lp.pool <= gb, "a plan within the limit");
 }
 
+// A small generator of shapes: t = 3..60000, N = 2^8..2^36, loads and k in use.
+struct Draw {
+    uint64_t s;
+    uint64_t operator()(uint64_t n) {
+        s = s * 6364136223846793005ULL + 1442695040888963407ULL;
+        return (s >> 33) % n;
+    }
+};
+
+cmc_params drawn(Draw& d) {
+    for (;;) {
+        const uint32_t t = uint32_t(3 + (d(64) << d(11)) % 60000), k = uint32_t(2 + d(3)), ell = uint32_t(8 + 4 * d(8));
+        const uint32_t load[] = {110, 125, 150, 220};
+        cmc_params p;
+        if (cmc_derive_params(uint32_t(1 + d(2)), t, ell, k, uint32_t(uint64_t(t) * load[d(4)] / 100) + 1, 100, 1, &p) == CMC_OK)
+            return p;
+    }
+}
+
+// A server plans its jobs at admission, for their size class and for each launch
+// with different counts: where the walk slots are and how many bytes are counted
+// must not depend on them, and what is admitted runs within the budget.
+void check_served_plans() {
+    Ctx c;
+    use_fake(c, 0);
+    Draw d{7};
+    const auto jobs_of = [&](const std::vector<cmc_params>& ps, uint32_t count) {
+        std::vector<Job> jobs(ps.size());
+        for (size_t i = 0; i < ps.size(); ++i)
+            require(c.make_job(ps[i], 0, count, 0, jobs[i]) == CMC_OK, "job");
+        return jobs;
+    };
+    for (int i = 0; i < 20000; ++i) {
+        const std::vector<cmc_params> one{drawn(d)};
+        Plan a, b;
+        uint64_t pa = 0, pb = 0;
+        require(c.plan_served(jobs_of(one, 1), ~0ull, false, a, pa) == CMC_OK &&
+                    c.plan_served(jobs_of(one, 200000), ~0ull, false, b, pb) == CMC_OK,
+                "plans");
+        require(a.slots_smem == b.slots_smem && pa == pb && a.claim_bytes == b.claim_bytes && a.ng == b.ng &&
+                    a.wg == b.wg && a.ns == b.ns,
+                "a served plan does not depend on the counts");
+        require(a.variant == 0 || a.claim_bytes == pa, "plain slots are counted as they are");
+        require(!a.reduced && a.claim_bytes <= pa, "item slots take no less than is counted");
+    }
+    const std::vector<cmc_params> wide{params(CMC_MODE_BGH25, 2000, 32, 3, 3000, 0)};
+    Plan pl;
+    uint64_t pool = 0;
+    require(c.plan_served(jobs_of(wide, 1), ~0ull, false, pl, pool) == CMC_OK && !pl.slots_smem &&
+                pl.claim_bytes > 600000000,
+            "t = 2000, N = 2^32 walks global slots and is counted so");
+
+    uint32_t shared = 0, fewer = 0;
+    for (int i = 0; i < 20000; ++i) {
+        std::vector<cmc_params> set;
+        for (uint64_t n = 1 + d(4); n; --n) set.push_back(drawn(d));
+        const uint64_t budget = (1 + d(1000)) << d(22);  // bytes for one of two iterations
+        require(c.plan_served(jobs_of(set, 1), budget, false, pl, pool) == CMC_OK, "plan");
+        if (pl.claim_bytes > budget) continue;  // not admitted
+        require(pool <= budget, "an admitted set's iteration is within the budget");
+        Plan rp;
+        uint64_t rpool = 0;
+        require(c.plan_served(jobs_of(set, 1), 2 * budget, true, rp, rpool) == CMC_OK && rpool <= 2 * budget,
+                "and so is its resident launch");
+        require(!rp.pool_stage, "resident launches have plain producers");
+        shared += rp.slots_smem;
+        fewer += rp.reduced;
+        for (const Plan* q : {&pl, &rp})
+            require(q->ng >= 1 && q->ns >= q->ng && q->ns % q->ng == 0 && q->smem_bytes <= 232448 && q->threads <= 512,
+                    "a plan that can be launched");
+        // each part of the set, in any proportion
+        std::vector<cmc_params> part{set[d(set.size())]};
+        if (set.size() > 2) part.push_back(set[0]);
+        require(c.plan_served(jobs_of(part, uint32_t(1 + d(1 << 20))), budget, false, pl, pool) == CMC_OK && pool <= budget,
+                "so is every part of an admitted set");
+    }
+    require(shared > 100 && fewer > 100, "budgets that bind");
+}
+
 }  // namespace
 
 int main() {
     const std::pair<const char*, void (*)()> tests[] = {{"buffers", check_grow}, {"graphs", check_graphs},
                                                         {"regions", check_regions},
-                                                        {"short memory", check_short_memory}};
+                                                        {"short memory", check_short_memory},
+                                                        {"served plans", check_served_plans}};
     int bad = 0;
     for (auto& [name, test] : tests) {
         try {
