@@ -122,11 +122,13 @@ typedef struct cmc_job {
 int cmc_run_jobs(cmc_ctx* ctx, const cmc_job* jobs, uint32_t njobs, uint64_t* out_failed,
                  uint32_t* out_offsets, uint32_t* out_jobs, uint64_t cap, uint64_t* out_total);
 
-/* Autotuner: times candidate plans (warps per table, walker isolation, map
- * method) on a sample of every job (first count/sample_div trials, at least
- * one), keeps the fastest for this mix of parameter sets, and applies it to
- * later cmc_run_jobs calls with the same mix.  *out_choice (may be NULL)
- * receives a description of the chosen plan. */
+/* Autotuner: times candidate plans of the group engine (warps per table, walker
+ * isolation, map method) on a sample of every job (first count/sample_div
+ * trials, at least one; 0: 64), and where one beats the automatic plan there,
+ * times both at the jobs' full counts.  A plan that wins there by 3 % is kept for
+ * this mix of parameter sets and applied to later cmc_run_jobs calls with the
+ * same mix and up to twice as many trials; other calls keep the automatic plan.
+ * *out_choice (may be NULL) receives a description of the chosen plan. */
 int cmc_autotune(cmc_ctx* ctx, const cmc_job* jobs, uint32_t njobs, uint32_t sample_div,
                  const char** out_choice);
 

@@ -110,6 +110,7 @@ struct TunedPlan {
     uint32_t wg = 0;
     int isolate = -1;
     int method = -1;
+    uint64_t trials = 0;  // of the call it was tuned for
 };
 
 struct Ctx {
