@@ -722,18 +722,23 @@ void Ctx::choose_engine(const std::vector<Job>& jobs, const Plan& group, LanePla
 // (64 sets of t = 16..4096 with 65,536 trials each: 2.6 GB, 6.6 with a region
 // for every class).
 int Ctx::plan_launch(const std::vector<Job>& jobs, const std::vector<uint32_t>& bounds, LaunchPlan& lp) {
-    lp = LaunchPlan{};
     const uint32_t nclass = uint32_t(bounds.size()) - 1;
     if (nclass < 1 || nclass > kMaxClasses) return fail(CMC_EINVAL, "bad plan classes");
-    lp.plans.resize(nclass);
-    lp.lanes.resize(nclass);
-    lp.waves.resize(nclass);
+    lp.plans.assign(nclass, Plan{});
+    lp.lanes.assign(nclass, LanePlan{});
+    lp.waves.assign(nclass, WavePlan{});
     lp.work.assign(nclass, 0.0);
     lp.trials.assign(nclass, 0.0);
     lp.region.assign(nclass, 0);
+    lp.kernels.clear();
+    lp.pool = 0;
+    lp.heaviest = 0;
+    lp.text.clear();
     bool any_split = false;
+    std::vector<Job> some;
     for (uint32_t c = 0; c < nclass; ++c) {
-        std::vector<Job> part(jobs.begin() + bounds[c], jobs.begin() + bounds[c + 1]);
+        if (nclass > 1) some.assign(jobs.begin() + bounds[c], jobs.begin() + bounds[c + 1]);
+        const std::vector<Job>& part = nclass > 1 ? some : jobs;
         const int rc = plan(part, lp.plans[c]);
         if (rc) return rc;
         any_split = any_split || lp.plans[c].walker_ctas;
@@ -743,7 +748,10 @@ int Ctx::plan_launch(const std::vector<Job>& jobs, const std::vector<uint32_t>& 
         }
         if (lp.trials[c] > lp.trials[lp.heaviest]) lp.heaviest = c;
         choose_engine(part, lp.plans[c], lp.lanes[c], lp.waves[c]);
-        lp.text += (c ? " | " : "") + plan_text + lanes_text(lp.lanes[c]) + waves_text(lp.waves[c]);
+        if (c) lp.text += " | ";
+        lp.text += plan_text;
+        if (lp.lanes[c].warps) lp.text += lanes_text(lp.lanes[c]);
+        if (lp.waves[c].ng) lp.text += waves_text(lp.waves[c]);
     }
     const bool fuse = use_fused && nclass > 1 && nclass <= kMaxFusedClasses && !any_split;
     if (fuse) lp.text = "fused(" + std::to_string(nclass) + ") " + lp.text;
@@ -834,7 +842,7 @@ int Ctx::run(const std::vector<Job>& jobs, uint64_t total, cudaStream_t st, uint
     cudaGetLastError();
     const std::vector<uint32_t> bounds = bounds_in ? *bounds_in : std::vector<uint32_t>{0, uint32_t(jobs.size())};
     const uint32_t nclass = uint32_t(bounds.size()) - 1;
-    LaunchPlan lp;
+    LaunchPlan& lp = call_plan;
     int rc = fit_launch(jobs, bounds, lp);
     if (rc) return rc;
     const std::vector<Plan>& plans = lp.plans;

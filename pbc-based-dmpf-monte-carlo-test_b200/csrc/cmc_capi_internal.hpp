@@ -145,6 +145,7 @@ struct Ctx {
     std::string err, plan_text;
     uint32_t kernels = 0;
     Plan last_plan;
+    LaunchPlan call_plan;  // of the last call: keeps its vectors' memory for the next
     Ctrl last_ctrl{};
     // tuning overrides (0 = automatic)
     uint32_t force_wg = 0, force_ng = 0, force_global_slots = 0, force_walkers = 0;
