@@ -219,7 +219,7 @@ __device__ __forceinline__ bool wave_map(const Job& J, const uint32_t* rec, cons
 // and branches).
 template <bool NARROW>
 __device__ __forceinline__ bool walk_bgh(const Job& J, bool active, uint64_t walk, uint64_t rnd, char* region,
-                                         uint32_t map_off, uint32_t& steps) {
+                                         uint32_t map_off, unsigned long long& probes) {
     // BGH25 random walk (cuckoo_core.hpp:123-133)
     using ItemT = Item<NARROW>;
     using Entry = typename ItemT::Entry;
@@ -246,7 +246,7 @@ __device__ __forceinline__ bool walk_bgh(const Job& J, bool active, uint64_t wal
         Entry old = mine;  // an item that returns to the bin it left finds the item that evicted it
         if (!again) old = ItemT::load(bins + bin);
         mine = it.pack(cur, which, four);
-        ++steps;
+        ++probes;
         which = digits.next(k);
         const bool placed = ItemT::empty(old);
         uint32_t copy;
@@ -260,7 +260,7 @@ __device__ __forceinline__ bool walk_bgh(const Job& J, bool active, uint64_t wal
         if (placed) ahead = ItemT::load(map + min(item + 1, last));
         failed = count > kick;
         if (which == copy && !failed) {
-            ++steps;
+            ++probes;
             const Entry back = it.pack(cur, which, four);
             it.unpack(mine, bin, four, cur, copy);
             mine = back;
@@ -277,7 +277,7 @@ __device__ __forceinline__ bool walk_bgh(const Job& J, bool active, uint64_t wal
 
 template <bool NARROW>
 __device__ __forceinline__ bool walk_drrt(const Job& J, bool active, char* region, uint32_t map_off,
-                                          uint32_t& steps) {
+                                          unsigned long long& probes) {
     // DRRT18 cycling eviction (cuckoo_core.hpp:134-158)
     using ItemT = Item<NARROW>;
     using Entry = typename ItemT::Entry;
@@ -298,7 +298,7 @@ __device__ __forceinline__ bool walk_drrt(const Job& J, bool active, char* regio
         if (!active) continue;
         const Entry old = ItemT::load(bins + bin);
         const Entry mine = it.pack(cur, which, four);
-        ++steps;
+        ++probes;
         const bool placed = ItemT::empty(old), evict = evicting && !placed;
         if (placed || (evict && count < kick)) ItemT::store(bins + bin, mine);
         active = !(placed && item == last);
@@ -446,14 +446,12 @@ __global__ void __launch_bounds__(512, 1) cmc_waves(const WaveArgs a) {
         const uint32_t job = owner ? __ldcg(mine + kStJob * 32) : 0u;
         const Job& J = a.jobs[job];
         char* region = regions + (uint64_t)min(own, n - 1) * a.region_bytes;
-        uint32_t steps = 0;
         bool failed = false;
         if (__any_sync(kFull, owner && J.mode == 1))
             failed = walk_bgh<NARROW>(J, owner && J.mode == 1, owner ? get64(kStWalk) : 0,
-                                      owner ? get64(kStWalk + 2) : 0, region, a.map_off, steps);
+                                      owner ? get64(kStWalk + 2) : 0, region, a.map_off, probes);
         if (__any_sync(kFull, owner && J.mode != 1))
-            failed = walk_drrt<NARROW>(J, owner && J.mode != 1, region, a.map_off, steps) || failed;
-        probes += steps;
+            failed = walk_drrt<NARROW>(J, owner && J.mode != 1, region, a.map_off, probes) || failed;
         if (owner) {
             ++walks;
             if (failed) {
