@@ -109,13 +109,16 @@ typedef struct cmc_job {
 } cmc_job;
 
 /* Batched form (no counterpart in the reference, which runs one parameter set
- * per process): all jobs in ONE persistent engine launch, heavy jobs first so
- * uneven table sizes balance across SMs.  Jobs whose best plans differ (walk
- * slots in shared or global memory, warps per group, entry width, cache kind)
- * form plan classes; each CTA runs one class at a time under that class's plan
- * and moves on to the class with the most work left when its own runs out.  out_failed[j] receives the number of
- * failing trials of job j.  If out_offsets is not NULL, the failing offsets are
- * written job by job in ascending order, out_jobs[i] (if not NULL) naming the
+ * per process): all jobs in one call, heavy jobs first so uneven table sizes
+ * balance across SMs.  Jobs whose best plans differ (walk slots in shared or
+ * global memory, warps per group, entry width, cache kind) form plan classes.
+ * Classes of the group engine with the same entry width and slot placement run
+ * in one persistent kernel, whose CTAs run one class at a time under that
+ * class's plan and move on to the class with the most work left when their own
+ * runs out; a class of the lane or wave engine, of pooled passes, or alone in its
+ * kind has a kernel of its own, one after another.  out_failed[j] receives the
+ * number of failing trials of job j.  If out_offsets is not NULL, the failing
+ * offsets are written job by job in ascending order, out_jobs[i] (if not NULL) naming the
  * job of out_offsets[i]; cap is their capacity and *out_total the number of
  * failures (when it exceeds cap, only the counts are complete).  Total trials
  * per call must be below 2^32.  Synchronous. */
@@ -275,7 +278,8 @@ double cmc_last_engine_ms(cmc_ctx* ctx);
 /* Counters of the last checked launch (cmc_launch, or cmc_check after
  * cmc_launch_device): out[0] walks, out[1] probes, out[2] cycles producer
  * groups waited for a free slot, out[3] cycles walker warps had nothing to
- * walk, out[4] walker warps' total cycles, out[5] device error code. */
+ * walk, out[4] walker warps' total cycles, out[5] device error code.  out[2..4]
+ * are the group engine's; the lane and wave engines have no such waits (0). */
 int cmc_last_stats(cmc_ctx* ctx, uint64_t out[6]);
 
 /* Kernels launched by the last cmc_launch* call on this context. */

@@ -207,16 +207,18 @@ __device__ __forceinline__ bool wave_map(const Job& J, const uint32_t* rec, cons
     return ok;
 }
 
-// The walks of a warp's trials, one per lane (`active`); returns whether this
-// lane's failed.  A step reads one bin per lane, all at the same place of the
-// loop, and its two outcomes (item placed, item evicted) are selects, not
-// branches.  A walk alone is bound by latency, the table read and the chain of
-// instructions behind it; beside other groups' fills by the ALU pipe, which
-// the fills use to 85 %.  The walk's digits are therefore decoded ahead, for
-// all lanes together, and an item that returns to the bin it left costs no
-// read (t = 1024, N = 2^20: 250 ALU instructions per step with 64-bit digit
-// divisions and a loop over returning items, 3,500 cycles a step with 32 lanes
-// and branches).
+// The walks of a warp's trials, one per lane (`active`), by the steps of ItemWalk
+// (cmc_trial.cuh), which the group engine uses: a change to the rules of a walk
+// has to be made in both.  Returns whether this lane's failed.
+//
+// A step reads one bin per lane, all at the same place of the loop, and its two
+// outcomes (item placed, item evicted) are selects, not branches.  A walk alone
+// is bound by latency, the table read and the chain of instructions behind it;
+// beside other groups' fills by the ALU pipe (79 % of a launch at t = 1024, under
+// ncu).  The walk's digits are therefore decoded ahead, for all lanes together,
+// and an item that returns to the bin it left costs no read (t = 1024, N = 2^20:
+// 250 ALU instructions per step with 64-bit digit divisions and a loop over
+// returning items, 3,500 cycles a step with 32 lanes and branches).
 template <bool NARROW>
 __device__ __forceinline__ bool walk_bgh(const Job& J, bool active, uint64_t walk, uint64_t rnd, char* region,
                                          uint32_t map_off, unsigned long long& probes) {
