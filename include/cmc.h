@@ -75,8 +75,9 @@ typedef struct cmc_ctx cmc_ctx;
  * device in the lane and wave engines (13 GB at t = 16384, 65,536 trials).  The
  * option "pool_bytes" bounds the tables and gives back what is above it.  A call
  * whose tables do not fit runs in the group engine with fewer walk slots; only
- * one that fits in no form fails (CMC_ENOMEM).  On a stream that is being
- * captured nothing is allocated: run the call, or a larger one, before. */
+ * one that fits in no form fails (CMC_ENOMEM).  On a stream that the caller
+ * captures nothing is allocated and the group engine runs: make the call, or a
+ * larger one, once before. */
 int cmc_init(int device, cmc_ctx** out);
 int cmc_destroy(cmc_ctx* ctx);
 const char* cmc_last_error(const cmc_ctx* ctx);

@@ -809,8 +809,13 @@ int Ctx::reserve_pool(uint64_t n) {
 // walk slots each time (t = 16384, B = 65535, 200 trials: 0.35 GB of waves, else
 // 12.4 GB of walk slots at most and 0.1 at least).
 int Ctx::fit_launch(const std::vector<Job>& jobs, const std::vector<uint32_t>& bounds, LaunchPlan& lp) {
+    // A graph that the caller captures names the pool for as long as it lives, and
+    // a later call may replace that: the group engine, which mostly needs none.
+    group_engine = fixed_memory && !capturing;
     int rc = plan_launch(jobs, bounds, lp);
-    if (rc || (rc = reserve_pool(lp.pool)) != CMC_ENOMEM) return rc;
+    if (!rc) rc = reserve_pool(lp.pool);
+    group_engine = false;
+    if (rc != CMC_ENOMEM) return rc;
     const std::string why = err;
     const uint64_t budget = slot_budget;
     uint64_t smallest = lp.pool;  // that was refused

@@ -213,11 +213,16 @@ void check_short_memory() {
                     require(pl.ng >= 1 && pl.ns >= pl.ng && pl.ns % pl.ng == 0, "slots for every group");
                 first = text;
             }
-            // under a capture the same plan, without a call
-            c.fixed_memory = true;
+            // under the call's own capture the same plan, and under the caller's
+            // the group engine; neither makes a call
             LaunchPlan lp;
+            const uint32_t calls = g_device.allocs + g_device.releases;
+            c.fixed_memory = c.capturing = true;
             require(fitted(c, *in, lp) == first, "the plan of a capture");
+            c.capturing = false;
+            require(!has(fitted(c, *in, lp), "->"), "no lanes or waves in the caller's graph");
             c.fixed_memory = false;
+            require(g_device.allocs + g_device.releases == calls, "no allocation during a capture");
             // more room: the engine of choice again
             g_device.size = 180 * gb;
             if (in != &wide) require(has(fitted(c, *in, lp), "->"), "memory that was short is not short for good");

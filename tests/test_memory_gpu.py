@@ -65,3 +65,39 @@ def test_a_limit_that_fits_nothing_is_refused(ctx, cmc):
     assert e.value.code == cmc.CMC_ENOMEM
     ctx.set_option("pool_bytes", 0)
     assert ctx.launch(p, cmc.batch_key(3, 1), 0, 200) == want
+
+
+@pytest.mark.parametrize("pool", ["none yet", "allocated"])
+def test_capture_of_a_device_launch_ends_well(cmc, pool):
+    # on a stream that the caller captures nothing is allocated, and the launch
+    # takes no tables that a later call could replace (the graph is not replayed)
+    import torch
+    p = cmc.parameters("bgh25", 64, 16, 3, 90, 40, "affine")
+    n = 1 << 17
+    key = torch.tensor(cmc.batch_key(3, 1), dtype=torch.int64).to(torch.int32).cuda()
+    offsets = torch.zeros(n, dtype=torch.int32, device="cuda")
+    nfailed = torch.zeros(1, dtype=torch.int32, device="cuda")
+    stream = torch.cuda.Stream()
+    with cmc.Context(0) as ctx:
+        def launch():
+            ctx.launch_device(p, key.data_ptr(), 0, n, offsets.data_ptr(), nfailed.data_ptr(), stream.cuda_stream)
+
+        if pool == "none yet":  # the other buffers are sized by a call in the group engine
+            ctx.set_option("lanes", 0)
+            ctx.set_option("waves", 0)
+        launch()
+        stream.synchronize()
+        ctx.check()
+        want = nfailed.item(), offsets[:nfailed.item()].tolist()
+        ctx.set_option("lanes", -1)
+        ctx.set_option("waves", -1)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            launch()
+        assert "-> engine" not in ctx.last_plan
+        del graph
+        launch()
+        stream.synchronize()
+        ctx.check()
+        assert "-> engine" in ctx.last_plan
+        assert (nfailed.item(), offsets[:nfailed.item()].tolist()) == want
